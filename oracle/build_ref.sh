@@ -10,7 +10,7 @@ set -euo pipefail
 REF="${GU_REFERENCE:-/root/reference}"
 HERE="$(cd "$(dirname "$0")" && pwd)"
 OUT="$HERE/_ref"
-if [ ! -d "$REF" ]; then
+if [ ! -f "$REF/parse.cpp" ]; then
   echo "build_ref: reference tree not present; skipping" >&2
   exit 0
 fi
