@@ -134,6 +134,18 @@ struct ChunkMap {
 // 2.84 ms; gu_graph_autotune also tries 0.06 and 1/3.
 constexpr float MS_RARE_FRAC = 0.15f;
 
+// Topological order of a directed acyclic graph (dag.cu), built on first use:
+// vertices by the length of their longest path to a sink, so every successor of
+// the vertex at position p sits at a position below p's level.
+struct TopoPlan {
+    enum State { UNBUILT, ACYCLIC, CYCLIC } state = UNBUILT;
+    int32_t *order = nullptr;  // [n] vertex at position p
+    int32_t *lvl = nullptr;    // [nlevels + 1] first position of each level
+    int32_t *PR = nullptr;     // [n + 1] out-edge offsets by position
+    int32_t *PC = nullptr;     // [m] positions of the successors
+    int nlevels = 0;
+};
+
 struct DeviceGraph {
     int device = 0;
     int32_t n = 0;
@@ -168,6 +180,7 @@ struct DeviceGraph {
     // BC work items over in-edges (forward) and out-edges (backward); for
     // undirected graphs bc_out aliases bc_in
     ChunkMap bc_in, bc_out;
+    TopoPlan topo;  // directed graphs
     std::vector<int32_t> host_R, host_RT;  // offsets kept on the host for building work items
     std::vector<void *> extra_allocs;  // freed with the graph
     // events bracketing the last main kernel launch (kernel-only timing): the

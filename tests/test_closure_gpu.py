@@ -1,0 +1,78 @@
+"""gu_dag_reach on bit rows at the edges of its chunks (4096 columns), column blocks
+(512 MiB of rows) and level structure, against the oracle's per-vertex set sizes.
+Counts are integers: the comparisons are exact."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import gu
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def closure(hg, stream=None):
+    g = gu.Graph(hg)
+    cnt = torch.full((max(hg.n, 1),), -5, dtype=torch.int64, device="cuda")
+    tot = g.dag_reach(cnt[: hg.n], stream=stream)
+    again = torch.full((max(hg.n, 1),), -7, dtype=torch.int64, device="cuda")
+    assert g.dag_reach(again[: hg.n]) == tot  # the kept order, a second time
+    np.testing.assert_array_equal(cnt.cpu().numpy()[: hg.n], again.cpu().numpy()[: hg.n])
+    return cnt.cpu().numpy()[: hg.n], tot
+
+
+@pytest.mark.parametrize("n,m", [(1, 0), (2, 1), (31, 60), (4095, 9000), (4096, 30000), (4097, 30000), (8193, 2000),
+                                 (70001, 280000)])
+def test_sizes_vs_oracle(n, m):
+    rng = np.random.default_rng(n)
+    a, b = rng.integers(0, n, m), rng.integers(0, n, m)
+    keep = a != b
+    perm = rng.permutation(n)
+    hg = gu.HostGraph.from_edges(n, perm[np.minimum(a, b)[keep]], perm[np.maximum(a, b)[keep]], symmetric=False)
+    counts, tot = closure(hg)
+    ref, rtot = oracle.dag_reach_counts(hg.R, hg.C, hg.n)
+    np.testing.assert_array_equal(counts, ref)
+    assert tot == rtot
+
+
+def test_path_star_and_empty():
+    n = 5000
+    path = gu.HostGraph.from_edges(n, np.arange(n - 1), np.arange(1, n), symmetric=False)  # 5000 levels
+    counts, tot = closure(path)
+    np.testing.assert_array_equal(counts, np.arange(n - 1, -1, -1))
+    star = gu.HostGraph.from_edges(n, np.zeros(n - 1, np.int32), np.arange(1, n), symmetric=False)  # one hub
+    counts, tot = closure(star)
+    assert tot == n - 1 and counts[0] == n - 1 and not counts[1:].any()
+    counts, tot = closure(gu.HostGraph(np.zeros(11, np.int32), np.zeros(0, np.int32), 10, True))
+    assert tot == 0 and not counts.any()
+
+
+def test_cycles_and_self_loops_keep_the_search():
+    """A directed graph with a cycle has no topological order: the counts are still the
+    numbers of other vertices reached, as the search from every vertex gives them."""
+    hg = gu.HostGraph.from_edges(300, np.arange(300), (np.arange(300) + 1) % 300, symmetric=False)
+    counts, tot = closure(hg)
+    assert tot == 300 * 299 and (counts == 299).all()
+    R = np.array([0, 2, 3, 3], np.int32)  # 0 -> 0, 0 -> 1, 1 -> 2
+    counts, tot = closure(gu.HostGraph(R, np.array([0, 1, 2], np.int32), 3, True))
+    np.testing.assert_array_equal(counts, [2, 1, 0])
+
+
+def test_no_memory_for_rows_falls_back():
+    hg = gu.HostGraph.dag(3000, 24000, seed=1)
+    ref, rtot = oracle.dag_reach_counts(hg.R, hg.C, hg.n)
+    g = gu.Graph(hg)
+    cnt = torch.empty(hg.n, dtype=torch.int64, device="cuda")
+    fail = gu.lib().gu_debug_fail_allocations
+    fail.argtypes = [ctypes.c_int64, ctypes.c_int64]
+    try:
+        # io staging, plan scratch and the order fit; both tries for the rows fail
+        assert fail(3, 2) == gu.OK
+        assert g.dag_reach(cnt) == rtot
+    finally:
+        fail(0, 0)
+    np.testing.assert_array_equal(cnt.cpu().numpy(), ref)
+    assert g.dag_reach(cnt) == rtot
+    np.testing.assert_array_equal(cnt.cpu().numpy(), ref)
