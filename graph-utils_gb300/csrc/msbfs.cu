@@ -793,9 +793,10 @@ __device__ void gather_mp(const MsArgs &a, const Lvl &L, const u64 *fmask = null
     const long long E = L.qedges;
     if (E == 0) return;
     const CtaQ cq{s_r + MP_STAGE, cq_count(), MP_QUEUE};
-    const long long per_blk = (E + G::nblk() - 1) / G::nblk();
-    const long long task = min((long long)MP_TASK, max(32ll, (per_blk + 31) & ~31ll));
-    const long long ntask = (E + task - 1) / task;
+    // (32-bit divisions: E is at most m, which is at most INT32_MAX)
+    const unsigned per_blk = ((unsigned)E + (unsigned)G::nblk() - 1u) / (unsigned)G::nblk();
+    const long long task = min((unsigned)MP_TASK, max(32u, (per_blk + 31u) & ~31u));
+    const long long ntask = ((unsigned)E + (unsigned)task - 1u) / (unsigned)task;
     for (long long t = G::blk(); t < ntask; t += G::nblk()) {
         const long long e0 = t * task;
         const long long e1 = min(E, e0 + task);
@@ -958,7 +959,7 @@ __device__ __forceinline__ void bu_found(const MsArgs &a, const Lvl &L, const Ct
 // scans only the vertices that still miss a source.
 __device__ __forceinline__ long long class_chunk(long long count, long long nwarps)
 {
-    return max(1ll, min(32ll, (count + nwarps - 1) / nwarps));
+    return max(1u, min(32u, ((unsigned)count + (unsigned)nwarps - 1u) / (unsigned)nwarps));
 }
 
 template <int W>
@@ -1612,9 +1613,11 @@ __device__ __forceinline__ void ms_search(const MsArgs &a, unsigned &epoch)
             if (VARIANT == GU_BFS_BOTTOM_UP) {
                 bu = j > 1;
             } else if (VARIANT == GU_BFS_AUTO) {
-                if (!prev_bu) bu = j > 1 && (double)L.qedges * (double)a.alpha > (double)a.m;
-                else bu = (double)L.qlen * (double)a.beta > (double)a.n &&
-                          (double)L.qedges * (double)a.gamma > (double)a.n;
+                // 32-bit floats: an SM of this part issues a warp's FP64 instruction over
+                // sixteen cycles, so a handful of them in each of its 32 warps would cost
+                // every level about a microsecond
+                if (!prev_bu) bu = j > 1 && (float)L.qedges * a.alpha > (float)a.m;
+                else bu = (float)L.qlen * a.beta > (float)a.n && (float)L.qedges * a.gamma > (float)a.n;
             }
             if (bu) {
                 // part A; F_0 may hold sources without in-edges, which no class list has
@@ -1680,7 +1683,7 @@ __device__ __forceinline__ void ms_search(const MsArgs &a, unsigned &epoch)
                 // only an OR of the frontier word into F_j (no read of seen, no
                 // first-discovery stamp), and one scan after the level keeps the
                 // bits not seen before, updates seen and builds the next queue.
-                L.scanq = VARIANT == GU_BFS_AUTO && (double)L.qedges > (double)a.n;
+                L.scanq = VARIANT == GU_BFS_AUTO && L.qedges > (long long)a.n;
                 td_update<W, G>(a, L);
                 if (VARIANT == GU_BFS_EDGE) gather_edge<W, G>(a, L);
                 else if (VARIANT == GU_BFS_WARP) gather_warp<W, G>(a, L);
