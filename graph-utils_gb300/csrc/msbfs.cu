@@ -521,7 +521,9 @@ __device__ __forceinline__ void flush_active(const Lvl &L, const u64 (&act)[W])
 template <int W, class G>
 __device__ void td_update(const MsArgs &a, const Lvl &L)
 {
-    const long long rank = G::rank(), size = G::size();
+    // From the last thread down: the gather that follows starts at the first CTA, so
+    // on a narrow level different CTAs do the two chains of dependent accesses.
+    const long long size = G::size(), rank = size - 1 - G::rank();
     u64 act[W] = {};
     for (long long i = rank; i < L.qlen; i += size) {
         const int32_t v = __ldcg(L.qcur + i);
