@@ -133,6 +133,7 @@ struct ChunkMap {
 // 1024 sources 1.465 -> 1.311 ms (0.06: 1.227), scale 22 x 256 sources 2.82 ->
 // 2.84 ms; gu_graph_autotune also tries 0.06 and 1/3.
 constexpr float MS_RARE_FRAC = 0.15f;
+constexpr float MS_ALPHA = 2.f;
 
 // Topological order of a directed acyclic graph (dag.cu), built on first use:
 // vertices by the length of their longest path to a sink, so every successor of
@@ -201,7 +202,7 @@ struct DeviceGraph {
 struct MsOptions {
     int variant = GU_BFS_AUTO;
     int batch_words = 0;  // 64-source words per batch (0: by the number of sources)
-    float alpha = 2.f;    // top-down -> bottom-up when frontier out-edges > m / alpha
+    float alpha = MS_ALPHA;  // top-down -> bottom-up when frontier out-edges > m / alpha
     float beta = 24.f;    // bottom-up -> top-down when frontier vertices < n / beta
     float gamma = 4.f;    // ... or when frontier out-edges < n / gamma
     // bottom-up levels expand top-down the sources that fewer than this fraction

@@ -1919,6 +1919,20 @@ static void launch_words(const MsArgs &a, int W, int sms, cudaStream_t stream, i
     else launch_one<V, 4>(a, sms, stream, max_blocks);
 }
 
+// Built-in direction settings of a graph, where neither its tuning nor the
+// environment gives them.  They weigh two fixed costs of a level against the work
+// that grows with the graph, so they go by its size:
+//   rare_frac  leaving rare sources to part C costs a barrier and a narrow top-down
+//              expansion, about 12 us; what it saves is scans of unreached vertices'
+//              lists.  Kernel times with 0.03 / 0.06 / 0.15 of the CTAs, 512 sources:
+//              R-MAT 16 434 / 456 / 518 us, 17 487 / 509 / 604, 18 657 / 628 / 689,
+//              19 1053 / 1015 / 1021, 20 1726 / 1737 / 1689.
+//   alpha      a bottom-up level takes two or three barriers, a top-down one takes
+//              one.  Alpha 1 / 2 (rare_frac 0), 150 sources: R-MAT 14 131 / 172 us,
+//              R-MAT 15 (ef 8) 149 / 178, R-MAT 16 (m = 1.8 M) 227 / 228, 17 370 / 204.
+static float ms_size_rare(float base, int32_t n) { return base * std::min(1.f, (float)n / (1 << 19)); }
+static float ms_size_alpha(float base, int64_t m) { return m < (1 << 20) ? 0.5f * base : base; }
+
 static float env_float(const char *name, float dflt)
 {
     const char *s = std::getenv(name);
@@ -1976,10 +1990,10 @@ void launch_msbfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t *di
     a.reach = opt.reach;
     a.ld = ld;
     ms_layout(ws, n, W, a);
-    a.alpha = opt.tuned ? opt.alpha : env_float("GU_MS_ALPHA", opt.alpha);
+    a.alpha = opt.tuned ? opt.alpha : env_float("GU_MS_ALPHA", ms_size_alpha(opt.alpha, g.m));
     a.beta = opt.tuned ? opt.beta : env_float("GU_MS_BETA", opt.beta);
     a.gamma = env_float("GU_MS_GAMMA", opt.gamma);
-    a.rare_frac = opt.tuned ? opt.rare_frac : env_float("GU_MS_RARE", opt.rare_frac);
+    a.rare_frac = opt.tuned ? opt.rare_frac : env_float("GU_MS_RARE", ms_size_rare(opt.rare_frac, g.n));
     int degbits = 1;
     while (degbits < 31 && (1ll << degbits) <= (long long)g.max_degree) ++degbits;
     a.degbits = degbits;
@@ -2103,10 +2117,12 @@ MsQueueLaunch launch_msbfs_queue(const std::vector<MsQueueRequest> &reqs, Worksp
     q.ws = ws;
     q.ws_stride = L.stride;
     q.group_size = L.group_size;
-    q.alpha = env_float("GU_MS_ALPHA", 2.f);
+    // a group's barrier is cheap next to the whole grid's: no size rule here (24 requests
+    // of the serving mix: 1429 us, with ms_size_alpha and ms_size_rare 1464 us)
+    q.alpha = env_float("GU_MS_ALPHA", MS_ALPHA);
     q.beta = env_float("GU_MS_BETA", 24.f);
     q.gamma = env_float("GU_MS_GAMMA", 4.f);
-    q.rare_frac = env_float("GU_MS_RARE", MsOptions().rare_frac);
+    q.rare_frac = env_float("GU_MS_RARE", MS_RARE_FRAC);
     q.wait_ns = wait_limit_ns();
     void *params[] = {&q};
     const void *fn = W == 1 ? (const void *)ms_queue_kernel<1> : W == 2 ? (const void *)ms_queue_kernel<2>
