@@ -367,7 +367,8 @@ gu_status gu_graph_last_launch(gu_graph g, double *kernel_seconds, int *td_level
         GU_CUDA_CHECK(cudaEventElapsedTime(&ms, dg.ev_start, dg.ev_stop));
         if (kernel_seconds) *kernel_seconds = ms / 1000.0;
         int err = 0, td = 0, bu = 0, ml = 0;
-        if (dg.ws.ptr) msbfs_read_status(dg, &err, &td, &bu, &ml);
+        if (dg.timeline == 2) smem_bfs_stats(dg, &td, &bu, &ml);
+        else if (dg.ws.ptr) msbfs_read_status(dg, &err, &td, &bu, &ml);
         if (td_levels) *td_levels = td;
         if (bu_levels) *bu_levels = bu;
         if (max_level) *max_level = ml;
@@ -402,6 +403,10 @@ gu_status gu_graph_level_profile(gu_graph g, int max_entries, int32_t *batch, in
         DeviceGraph &dg = *g->g;
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
+        if (dg.timed && dg.timeline == 2) {  // the shared-memory engine keeps no phase timeline
+            if (count) *count = 0;
+            return;
+        }
         if (!dg.timed || !dg.ws.ptr) throw gu_error(GU_ERR_INVALID_ARGUMENT, "no launch recorded on this graph yet");
         GU_CUDA_CHECK(cudaEventSynchronize(dg.ev_stop));
         const int c = dg.timeline == 1
@@ -418,6 +423,11 @@ gu_status gu_graph_level_idle(gu_graph g, int max_entries, double *idle_cta_ms, 
         DeviceGraph &dg = *g->g;
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
+        if (dg.timed && dg.timeline == 2) {
+            if (nblocks) *nblocks = 0;
+            if (count) *count = 0;
+            return;
+        }
         if (!dg.timed || !dg.ws.ptr || dg.timeline == 1)
             throw gu_error(GU_ERR_INVALID_ARGUMENT, "no batched search recorded on this graph yet");
         GU_CUDA_CHECK(cudaEventSynchronize(dg.ev_stop));
@@ -457,7 +467,7 @@ static void bfs_device(DeviceGraph &g, int variant, const int32_t *sources_dev, 
     }
     MsOptions opt;
     opt.variant = variant;
-    if (variant == GU_BFS_AUTO && g.tune.set) {  // the measured choice (gu_graph_autotune)
+    if (variant == GU_BFS_AUTO && g.tune.set && g.tune.engine != GU_ENGINE_SHARED) {  // the measured choice
         if (g.tune.engine == GU_ENGINE_PER_SOURCE &&
             launch_local_bfs(g, sources_dev, k, dist_dev, ld, nullptr, nullptr, stream))
             return;
@@ -476,15 +486,10 @@ static void bfs_device(DeviceGraph &g, int variant, const int32_t *sources_dev, 
             opt.tuned = true;
         }
     } else if (variant == GU_BFS_AUTO) {
-        const AutoEngine eng = auto_engine(g, true);
-        if (eng == AutoEngine::LOCAL && launch_local_bfs(g, sources_dev, k, dist_dev, ld, nullptr, nullptr, stream))
+        if (launch_smem_bfs(g, sources_dev, k, dist_dev, ld, nullptr, nullptr, stream)) return;
+        if (!smem_bfs_takes(g, k) && auto_engine(g) == AutoEngine::LOCAL &&
+            launch_local_bfs(g, sources_dev, k, dist_dev, ld, nullptr, nullptr, stream))
             return;
-        if (eng == AutoEngine::PLAIN) {
-            launch_plain_bfs(g, sources_dev, k, dist_dev, ld, stream);
-            GU_CUDA_CHECK(cudaStreamSynchronize(stream));
-            GU_CUDA_CHECK(cudaGetLastError());
-            return;
-        }
     }
     launch_msbfs(g, sources_dev, k, dist_dev, ld, opt, stream, nullptr);
     check_dev_status(g, stream);
@@ -540,6 +545,7 @@ gu_status gu_graph_autotune(gu_graph g, const int32_t *sources_dev, int32_t k, g
         };
         if (dg.max_degree <= 16) add(GU_ENGINE_PER_SOURCE, 0, 0, 0);
         if (dg.n <= 65536) add(GU_ENGINE_ONE_CTA, 0, 0, 0);
+        if (smem_bfs_takes(dg, k)) add(GU_ENGINE_SHARED, 0, 0, 0);
         const int wd = msbfs_words_for(k);
         const float grid[][2] = {{2.f, 24.f}, {1.f, 24.f}, {4.f, 24.f}, {8.f, 24.f}, {2.f, 12.f}, {2.f, 48.f}};
         for (int w = wd; w >= 1 && w >= wd / 2; w /= 2) {
@@ -614,7 +620,7 @@ gu_status gu_graph_set_tuning(gu_graph g, const gu_tuning *t)
             dg.tune = DeviceGraph::Tuning();
             return;
         }
-        if (t->engine < GU_ENGINE_BATCHED || t->engine > GU_ENGINE_ONE_CTA)
+        if (t->engine < GU_ENGINE_BATCHED || t->engine > GU_ENGINE_SHARED)
             throw gu_error(GU_ERR_INVALID_ARGUMENT, "unknown engine");
         if (t->engine == GU_ENGINE_PER_SOURCE && dg.max_degree > 16)
             throw gu_error(GU_ERR_INVALID_ARGUMENT, "the per-source engine needs out-degree <= 16");
@@ -653,13 +659,14 @@ gu_status gu_bfs(gu_graph g, int variant, const int32_t *sources_dev, int32_t k,
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
         // Source ids are checked before they index anything: by the batched kernel
-        // itself where it is the engine that runs (it skips a bad id and reports it
-        // as GU_ERR_INVALID_ARGUMENT), else here on the host, which costs a copy and a
+        // and the shared-memory one themselves (they skip a bad id and report it as
+        // GU_ERR_INVALID_ARGUMENT), else here on the host, which costs a copy and a
         // synchronisation per call.
         const bool batched = variant != GU_BFS_PLAIN &&
                              (variant != GU_BFS_AUTO ||
-                              (dg.tune.set ? dg.tune.engine == GU_ENGINE_BATCHED
-                                           : auto_engine(dg, true) == AutoEngine::BATCHED));
+                              (dg.tune.set && dg.tune.engine != GU_ENGINE_SHARED
+                                   ? dg.tune.engine == GU_ENGINE_BATCHED
+                                   : smem_bfs_takes(dg, k) || auto_engine(dg) == AutoEngine::BATCHED));
         if (!batched && k > 0) {
             std::vector<int32_t> hs((size_t)k);
             GU_CUDA_CHECK(cudaMemcpyAsync(hs.data(), sources_dev, sizeof(int32_t) * (size_t)k, cudaMemcpyDeviceToHost,
@@ -946,8 +953,9 @@ gu_status gu_diameter(gu_graph g, const int32_t *sources_dev, int32_t k, int32_t
         *diameter = 0;
         if (k == 0) return;
         int ml = 0;
-        if (auto_engine(dg, false) == AutoEngine::LOCAL &&
-            launch_local_bfs(dg, sources_dev, k, nullptr, dg.n, nullptr, &ml, st)) {
+        if (launch_smem_bfs(dg, sources_dev, k, nullptr, dg.n, nullptr, &ml, st) ||
+            (auto_engine(dg) == AutoEngine::LOCAL &&
+             launch_local_bfs(dg, sources_dev, k, nullptr, dg.n, nullptr, &ml, st))) {
             *diameter = ml;
             return;
         }
@@ -1004,9 +1012,10 @@ gu_status gu_reach(gu_graph g, const int32_t *sources_dev, int32_t k, int64_t *c
         cudaStream_t st = (cudaStream_t)stream;
         check_sources_device(dg, sources_dev, k, st);
         if (k == 0) return;
-        GU_CUDA_CHECK(cudaMemsetAsync(counts_dev, 0, sizeof(int64_t) * (size_t)k, st));
         auto *cnt = reinterpret_cast<unsigned long long *>(counts_dev);
-        if (auto_engine(dg, false) == AutoEngine::LOCAL &&
+        if (launch_smem_bfs(dg, sources_dev, k, nullptr, dg.n, cnt, nullptr, st)) return;
+        GU_CUDA_CHECK(cudaMemsetAsync(counts_dev, 0, sizeof(int64_t) * (size_t)k, st));
+        if (auto_engine(dg) == AutoEngine::LOCAL &&
             launch_local_bfs(dg, sources_dev, k, nullptr, dg.n, cnt, nullptr, st))
             return;
         GU_CUDA_CHECK(cudaMemsetAsync(counts_dev, 0, sizeof(int64_t) * (size_t)k, st));

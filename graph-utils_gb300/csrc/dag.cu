@@ -364,7 +364,7 @@ static void reach_by_search(DeviceGraph &g, unsigned long long *cnt, char *io, c
     int32_t *src = reinterpret_cast<int32_t *>(io + 256);
     iota_kernel<<<blocks, 256, 0, st>>>(src, g.n);
     GU_CUDA_CHECK(cudaGetLastError());
-    if (auto_engine(g, false) == AutoEngine::LOCAL && launch_local_bfs(g, src, g.n, nullptr, g.n, cnt, nullptr, st)) return;
+    if (auto_engine(g) == AutoEngine::LOCAL && launch_local_bfs(g, src, g.n, nullptr, g.n, cnt, nullptr, st)) return;
     GU_CUDA_CHECK(cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (size_t)g.n, st));
     MsOptions opt;
     opt.variant = GU_BFS_AUTO;

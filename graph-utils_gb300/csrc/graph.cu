@@ -192,6 +192,7 @@ DeviceGraph::~DeviceGraph()
         if (ring_stop[i]) cudaEventDestroy(ring_stop[i]);
     }
     if (ctl_host) cudaFreeHost(ctl_host);
+    if (sb_status) cudaFreeHost(sb_status);
     if (copy_st) cudaStreamDestroy(copy_st);
     ws.release();
     io.release();
@@ -227,6 +228,10 @@ void ensure_coo(DeviceGraph &g, cudaStream_t stream)
     GU_CUDA_CHECK(cudaGetLastError());
 }
 
+// Adjacency arrays are allocated in whole 32-byte sectors: a list may be read by
+// the aligned sector.
+static size_t adjacency_bytes(int64_t m) { return sizeof(int32_t) * (((size_t)(m > 0 ? m : 1) + 7) & ~(size_t)7); }
+
 DeviceGraph *create_device_graph(const int32_t *R, const int32_t *C, int32_t n, int64_t m, bool directed,
                                  cudaStream_t stream)
 {
@@ -259,7 +264,7 @@ DeviceGraph *create_device_graph(const int32_t *R, const int32_t *C, int32_t n, 
     sort_adjacency_by_key(R, Cs.data(), n, outdeg.data());
     g->host_R.assign(R, R + n + 1);
     GU_CUDA_CHECK(dev_malloc((void **)&g->R, sizeof(int32_t) * ((size_t)n + 1)));
-    GU_CUDA_CHECK(dev_malloc((void **)&g->C, sizeof(int32_t) * (size_t)(m > 0 ? m : 1)));
+    GU_CUDA_CHECK(dev_malloc((void **)&g->C, adjacency_bytes(m)));
     GU_CUDA_CHECK(cudaMemcpyAsync(g->R, R, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, stream));
     if (m > 0) GU_CUDA_CHECK(cudaMemcpyAsync(g->C, Cs.data(), sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, stream));
     g->bytes = sizeof(int32_t) * ((size_t)n + 1 + (size_t)m);
@@ -272,7 +277,7 @@ DeviceGraph *create_device_graph(const int32_t *R, const int32_t *C, int32_t n, 
         sort_adjacency_by_key(t.R.data(), t.C.data(), n, outdeg.data());
         g->host_RT = t.R;
         GU_CUDA_CHECK(dev_malloc((void **)&g->RT, sizeof(int32_t) * ((size_t)n + 1)));
-        GU_CUDA_CHECK(dev_malloc((void **)&g->CT, sizeof(int32_t) * (size_t)(m > 0 ? m : 1)));
+        GU_CUDA_CHECK(dev_malloc((void **)&g->CT, adjacency_bytes(m)));
         GU_CUDA_CHECK(cudaMemcpyAsync(g->RT, t.R.data(), sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, stream));
         if (m > 0) GU_CUDA_CHECK(cudaMemcpyAsync(g->CT, t.C.data(), sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, stream));
         GU_CUDA_CHECK(cudaStreamSynchronize(stream));  // t goes out of scope

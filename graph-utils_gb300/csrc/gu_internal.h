@@ -26,6 +26,8 @@ namespace gu {
 constexpr int BU_LIGHT_DEGREE = 8;
 constexpr int BU_MID_DEGREE = 32;
 constexpr int BU_HEAVY_DEGREE = 128;
+// AUTO takes the per-source engine with shared-memory queues up to this out-degree.
+constexpr int LOCAL_MAX_DEGREE = 16;
 // Every workspace starts with this many bytes of launch control block and
 // profiling timeline; kernel scratch follows.
 constexpr size_t WS_CONTROL_BYTES = 65536;
@@ -165,6 +167,9 @@ struct DeviceGraph {
         int ctas_per_sm = 0;  // batched engine's grid: CTAs per SM (0: as many as fit)
         float rare_frac = MS_RARE_FRAC;
     } tune;
+    void *sb_head = nullptr;    // shared-memory engine: first in-neighbours, built on first use
+    void *sb_status = nullptr;  // shared-memory engine: its clusters' reports (pinned)
+    int sb_clusters = 0;        // ... of the last launch
     void *ctl_host = nullptr;  // pinned copy of the batched engine's control block, written after each launch
     int32_t *ell = nullptr;  // low-degree graphs: neighbours padded to ell_width per vertex (-1), built on first use
     int ell_width = 0;
@@ -192,7 +197,7 @@ struct DeviceGraph {
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     cudaStream_t copy_st = nullptr;  // host-form calls copy rows out on it while later sources run
     bool timed = false;
-    int timeline = 0;  // engine whose phase timeline the workspace holds: 0 batched BFS, 1 BC
+    int timeline = 0;  // engine whose phase timeline the workspace holds: 0 batched BFS, 1 BC; 2: none (shared-memory engine)
     void mark_start(cudaStream_t s);
     void mark_stop(cudaStream_t s);
     ~DeviceGraph();
@@ -236,10 +241,17 @@ void launch_plain_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
 // Reachable-set sizes of every vertex of a DAG (self excluded) and their sum.
 void dag_reach(DeviceGraph &g, int64_t *counts, int64_t *total_host, cudaStream_t st);
 int msbfs_words_for(int32_t k);  // 64-source words per batch for k sources
-enum class AutoEngine { LOCAL, PLAIN, BATCHED };
-AutoEngine auto_engine(const DeviceGraph &g, bool rows);
+enum class AutoEngine { LOCAL, BATCHED };
+AutoEngine auto_engine(const DeviceGraph &g);
 bool launch_local_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t *dist, int64_t ld,
                       unsigned long long *reach, int *max_level_host, cudaStream_t stream);
+// Shared-memory engine (smem.cu): whether AUTO takes it for k sources; rows (dist
+// non-null) and / or counts.  Checks the sources on the device; synchronises; false
+// means that another engine runs the search.
+bool smem_bfs_takes(const DeviceGraph &g, int32_t k);
+bool launch_smem_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t *dist, int64_t ld,
+                     unsigned long long *reach, int *max_level, cudaStream_t stream);
+void smem_bfs_stats(const DeviceGraph &g, int *td_levels, int *bu_levels, int *max_level);
 // Batched sigma / Brandes: bc (n doubles, may be null), optional rows (k x ld).
 void launch_bc(DeviceGraph &g, const int32_t *sources, int32_t k, const BcOptions &opt, double *bc, int32_t *dist_rows,
                uint64_t *sigma_rows, double *delta_rows, int64_t ld, bool backward, cudaStream_t stream);

@@ -42,8 +42,6 @@ namespace gu {
 // 1024 threads and two 6144-vertex queues, and no less with smaller queues.
 constexpr int LOCAL_THREADS = 1024;
 constexpr int LOCAL_QCAP = 6144;      // vertices per shared-memory level queue (two queues: 48 KiB)
-constexpr int LOCAL_MAX_DEGREE = 16;     // AUTO takes this engine up to this out-degree
-constexpr int PLAIN_MAX_VERTICES = 4096;  // ... and the one-CTA-per-source form up to this many vertices
 constexpr size_t LOCAL_SMEM = 2 * LOCAL_QCAP * sizeof(int32_t);
 
 struct LocalArgs {
@@ -164,19 +162,16 @@ __global__ void __launch_bounds__(LOCAL_THREADS, 2) local_bfs_kernel(LocalArgs a
     }
 }
 
-// AUTO's engine choice: the per-source engine for low-degree graphs (its
-// thread-per-vertex expansion wants short adjacency lists), the one-CTA-per-
-// source warp-per-vertex form for tiny graphs with longer lists (distance rows
-// only: it has no counting mode), the batched bit-matrix engine otherwise.
+// AUTO's choice where the shared-memory engine (smem.cu) does not apply: the
+// per-source engine for low-degree graphs (its thread-per-vertex expansion wants
+// short adjacency lists), the batched bit-matrix engine otherwise.
 // GU_AUTO_LOCAL=0 in the environment keeps AUTO on the batched engine (tests use
 // it to cover every engine on the same graphs).
-AutoEngine auto_engine(const DeviceGraph &g, bool rows)
+AutoEngine auto_engine(const DeviceGraph &g)
 {
     const char *e = std::getenv("GU_AUTO_LOCAL");
     if (e && e[0] == '0') return AutoEngine::BATCHED;
-    if (g.max_degree <= LOCAL_MAX_DEGREE) return AutoEngine::LOCAL;
-    if (rows && g.n <= PLAIN_MAX_VERTICES) return AutoEngine::PLAIN;
-    return AutoEngine::BATCHED;
+    return g.max_degree <= LOCAL_MAX_DEGREE ? AutoEngine::LOCAL : AutoEngine::BATCHED;
 }
 
 // Returns false if a frontier overflowed the shared queues (the caller reruns the
@@ -233,6 +228,7 @@ bool launch_local_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
     a.max_level = reinterpret_cast<int *>(ws);
     a.overflow = reinterpret_cast<int *>(ws) + 1;
     a.qcap = qcap;
+    g.timeline = 0;
     g.mark_start(stream);
     kern<<<grid, LOCAL_THREADS, smem, stream>>>(a);
     GU_CUDA_CHECK(cudaGetLastError());

@@ -92,6 +92,7 @@ void launch_plain_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
     int32_t *qbuf = reinterpret_cast<int32_t *>(ws + WS_CONTROL_BYTES);
     // no level statistics or timeline for this form
     GU_CUDA_CHECK(cudaMemsetAsync(ws, 0, WS_CONTROL_BYTES, stream));
+    g.timeline = 0;
     g.mark_start(stream);
     plain_bfs_kernel<<<grid, PLAIN_THREADS, 0, stream>>>(g.R, g.C, g.n, sources, k, dist, ld, qbuf);
     GU_CUDA_CHECK(cudaGetLastError());

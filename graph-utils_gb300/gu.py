@@ -36,7 +36,7 @@ class GuTuning(ctypes.Structure):
                 ("seconds", ctypes.c_double)]
 
 
-ENGINES = {0: "batched", 1: "per-source", 2: "one-cta"}
+ENGINES = {0: "batched", 1: "per-source", 2: "one-cta", 3: "shared-memory"}
 RARE_FRAC = 0.15  # the batched engine's default rare-source fraction (gu_tuning.rare_frac)
 
 

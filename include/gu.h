@@ -48,13 +48,14 @@ typedef enum gu_status {
  *   SCAN      block-scan ranked gather     (multi_search/scan_based.cu:43-194)
  *   SHUFFLE   warp per vertex, dynamic queue (multi_search/shuffle_based.cuh:81-286)
  *   BOTTOM_UP frontier bitmap pull (no reference counterpart)
- *   AUTO      engine by graph shape -- per-source BFS with shared-memory queues
- *             for out-degree <= 16 (meshes; falls back on frontier overflow), the
- *             PLAIN form for n <= 4096, else the batched engine with per-level
- *             direction and gather choice
+ *   AUTO      engine by graph shape and source count -- one cluster of CTAs per
+ *             source with bitmaps in shared memory for small graphs and few
+ *             sources, per-source BFS with shared-memory queues for out-degree
+ *             <= 16 (meshes; falls back on frontier overflow), else the batched
+ *             engine with per-level direction and gather choice
  *   PLAIN     one CTA per source, int32 distance row as the visited set -- the
  *             reference's own structure, kept as the one-launch-per-request baseline.
- * All but PLAIN run 64 sources per bitmap word in one persistent launch. */
+ * The others run 64 sources per bitmap word in one persistent launch. */
 typedef enum gu_bfs_variant {
     GU_BFS_AUTO = 0,
     GU_BFS_LINEAR = 1,
@@ -213,7 +214,8 @@ gu_status gu_graph_level_idle(gu_graph g, int max_entries, double *idle_cta_ms, 
  * by its kernel, and makes the fastest the graph's AUTO choice for later gu_bfs
  * / gu_bfs_host calls (the server and the counting calls keep the built-in
  * choice).  Candidates: the per-source engine (out-degree <= 16), the
- * one-CTA-per-source form (n <= 65536), and the batched engine over a grid of
+ * one-CTA-per-source form (n <= 65536), the shared-memory engine (where AUTO takes
+ * it for k sources), and the batched engine over a grid of
  * direction thresholds (alpha: top-down -> bottom-up when the frontier's
  * out-edges exceed m / alpha; beta: back when the frontier holds fewer than
  * n / beta vertices), source words per batch and the persistent grid's CTAs
@@ -224,7 +226,9 @@ gu_status gu_graph_level_idle(gu_graph g, int max_entries, double *idle_cta_ms, 
 typedef enum gu_engine {
     GU_ENGINE_BATCHED = 0,    /* bit-matrix engine, 64 x words sources per batch */
     GU_ENGINE_PER_SOURCE = 1, /* one CTA per source, shared-memory level queues */
-    GU_ENGINE_ONE_CTA = 2     /* PLAIN: one CTA per source, distance row as visited set */
+    GU_ENGINE_ONE_CTA = 2,    /* PLAIN: one CTA per source, distance row as visited set */
+    GU_ENGINE_SHARED = 3      /* one cluster of CTAs per source, state in shared memory (where AUTO would
+                                 take it; elsewhere AUTO's other engines run) */
 } gu_engine;
 
 typedef struct gu_tuning {
