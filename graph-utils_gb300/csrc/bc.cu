@@ -900,6 +900,12 @@ static int bc_words_for(int32_t k, int requested)
     return W;
 }
 
+void check_bc_batch(int32_t k, int32_t batch)
+{
+    if (batch > 0 && batch % 64) throw gu_error(GU_ERR_INVALID_ARGUMENT, "batch must be a multiple of 64");
+    if (batch > 0) (void)bc_words_for(k, batch / 64);
+}
+
 static DevChunks dev_chunks(const ChunkMap &c)
 {
     DevChunks d;

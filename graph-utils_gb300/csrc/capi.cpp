@@ -368,6 +368,7 @@ gu_status gu_graph_last_launch(gu_graph g, double *kernel_seconds, int *td_level
         if (kernel_seconds) *kernel_seconds = ms / 1000.0;
         int err = 0, td = 0, bu = 0, ml = 0;
         if (dg.timeline == 2) smem_bfs_stats(dg, &td, &bu, &ml);
+        else if (dg.timeline == 3) ml = dg.sc_levels;
         else if (dg.ws.ptr) msbfs_read_status(dg, &err, &td, &bu, &ml);
         if (td_levels) *td_levels = td;
         if (bu_levels) *bu_levels = bu;
@@ -403,7 +404,7 @@ gu_status gu_graph_level_profile(gu_graph g, int max_entries, int32_t *batch, in
         DeviceGraph &dg = *g->g;
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
-        if (dg.timed && dg.timeline == 2) {  // the shared-memory engine keeps no phase timeline
+        if (dg.timed && dg.timeline >= 2) {  // the shared-memory engines keep no phase timeline
             if (count) *count = 0;
             return;
         }
@@ -428,7 +429,7 @@ gu_status gu_graph_level_idle(gu_graph g, int max_entries, double *idle_cta_ms, 
             if (count) *count = 0;
             return;
         }
-        if (!dg.timed || !dg.ws.ptr || dg.timeline == 1)
+        if (!dg.timed || !dg.ws.ptr || dg.timeline == 1 || dg.timeline == 3)
             throw gu_error(GU_ERR_INVALID_ARGUMENT, "no batched search recorded on this graph yet");
         GU_CUDA_CHECK(cudaEventSynchronize(dg.ev_stop));
         const int c = msbfs_read_idle(dg, max_entries, idle_cta_ms, nblocks);
@@ -754,6 +755,10 @@ gu_status gu_sigma(gu_graph g, const int32_t *sources_dev, int32_t k, int32_t *d
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
         cudaStream_t st = (cudaStream_t)stream;
+        if (k > 0 && sources_dev && smem_bc_takes(dg, k, 0)) {
+            launch_smem_bc(dg, sources_dev, k, nullptr, dist_dev, sigma_dev, nullptr, ld, st);
+            return;
+        }
         check_sources_device(dg, sources_dev, k, st);
         if (k == 0) return;
         BcOptions opt;
@@ -773,6 +778,11 @@ gu_status gu_bc(gu_graph g, const int32_t *sources_dev, int32_t k, int32_t batch
         std::lock_guard<std::mutex> lk(dg.mu);
         DeviceScope ds(dg.device);
         cudaStream_t st = (cudaStream_t)stream;
+        if (k > 0 && sources_dev && smem_bc_takes(dg, k, batch)) {
+            check_bc_batch(k, batch);
+            launch_smem_bc(dg, sources_dev, k, bc_dev, nullptr, nullptr, delta_dev, ld, st);
+            return;
+        }
         check_sources_device(dg, sources_dev, k, st);
         if (k == 0) {
             GU_CUDA_CHECK(cudaMemsetAsync(bc_dev, 0, sizeof(double) * (size_t)dg.n, st));

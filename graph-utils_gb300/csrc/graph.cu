@@ -193,6 +193,7 @@ DeviceGraph::~DeviceGraph()
     }
     if (ctl_host) cudaFreeHost(ctl_host);
     if (sb_status) cudaFreeHost(sb_status);
+    if (sc_report) cudaFreeHost(sc_report);
     if (copy_st) cudaStreamDestroy(copy_st);
     ws.release();
     io.release();

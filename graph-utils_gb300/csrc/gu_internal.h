@@ -170,6 +170,10 @@ struct DeviceGraph {
     void *sb_head = nullptr;    // shared-memory engine: first in-neighbours, built on first use
     void *sb_status = nullptr;  // shared-memory engine: its clusters' reports (pinned)
     int sb_clusters = 0;        // ... of the last launch
+    void *sc_graph = nullptr;   // shared-memory BC engine: the graph renumbered, 16-bit ids, built on first use
+    int32_t sc_nlong = 0;       // ... its vertices with long lists
+    void *sc_report = nullptr;  // ... and its CTAs' reports (pinned)
+    int sc_levels = 0;          // ... deepest level of its last launch
     void *ctl_host = nullptr;  // pinned copy of the batched engine's control block, written after each launch
     int32_t *ell = nullptr;  // low-degree graphs: neighbours padded to ell_width per vertex (-1), built on first use
     int ell_width = 0;
@@ -197,7 +201,7 @@ struct DeviceGraph {
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     cudaStream_t copy_st = nullptr;  // host-form calls copy rows out on it while later sources run
     bool timed = false;
-    int timeline = 0;  // engine whose phase timeline the workspace holds: 0 batched BFS, 1 BC; 2: none (shared-memory engine)
+    int timeline = 0;  // engine whose phase timeline the workspace holds: 0 batched BFS, 1 BC; 2, 3: none (shared-memory BFS, BC)
     void mark_start(cudaStream_t s);
     void mark_stop(cudaStream_t s);
     ~DeviceGraph();
@@ -255,6 +259,13 @@ void smem_bfs_stats(const DeviceGraph &g, int *td_levels, int *bu_levels, int *m
 // Batched sigma / Brandes: bc (n doubles, may be null), optional rows (k x ld).
 void launch_bc(DeviceGraph &g, const int32_t *sources, int32_t k, const BcOptions &opt, double *bc, int32_t *dist_rows,
                uint64_t *sigma_rows, double *delta_rows, int64_t ld, bool backward, cudaStream_t stream);
+// Small graphs, one CTA per source (smem_bc.cu): whether gu_bc / gu_sigma take it; bc
+// null: counts only.  Checks the sources on the device; synchronises.
+bool smem_bc_takes(const DeviceGraph &g, int32_t k, int32_t batch);
+void launch_smem_bc(DeviceGraph &g, const int32_t *sources, int32_t k, double *bc, int32_t *dist_rows,
+                    uint64_t *sigma_rows, double *delta_rows, int64_t ld, cudaStream_t stream);
+// Throws GU_ERR_INVALID_ARGUMENT for a batch that gu_bc does not take.
+void check_bc_batch(int32_t k, int32_t batch);
 size_t bc_workspace_bytes(const DeviceGraph &g, int32_t k, int batch, bool backward);
 // One request of a work-queue launch: BFS rows (dist, k x ld) and/or reachable
 // counts (reach, k) of k sources on graph g (any graph on the current device).

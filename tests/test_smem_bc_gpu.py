@@ -1,0 +1,109 @@
+"""gu_bc and gu_sigma on small graphs (one CTA per source, state in shared memory) at the
+edges of their sizes and list lengths: counts and distances exact, dependencies and
+betweenness within 1e-12 relative of the FP64 oracle, equal bits on a second call."""
+import numpy as np
+import pytest
+
+import gu
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+RTOL = 1e-12
+
+
+def check(hg, srcs, directed=False):
+    g = gu.Graph(hg)
+    n, k = hg.n, len(srcs)
+    s = torch.as_tensor(np.asarray(srcs, np.int32), device="cuda")
+    sig = torch.full((k, n), -7, dtype=torch.int64, device="cuda")
+    d = torch.full((k, n), -7, dtype=torch.int32, device="cuda")
+    g.sigma(s, sig, dist_dev=d)
+    assert g.level_profile() == []  # no phase timeline: this engine ran
+    rd, rs = oracle.sigma_multi(hg.R, hg.C, n, srcs, nthreads=8)
+    np.testing.assert_array_equal(d.cpu().numpy(), rd)
+    np.testing.assert_array_equal(sig.cpu().numpy().view(np.uint64), rs)
+    bc = torch.empty(n, dtype=torch.float64, device="cuda")
+    delta = torch.full((k, n), -7.0, dtype=torch.float64, device="cuda")
+    g.bc(s, bc, delta_dev=delta)
+    assert g.last_launch()[3] == rd[rd != gu.UNREACHABLE].max()
+    again = torch.empty_like(bc)
+    g.bc(s, again)
+    assert torch.equal(bc.view(torch.int64), again.view(torch.int64))
+    np.testing.assert_allclose(bc.cpu().numpy(), oracle.bc(hg.R, hg.C, n, srcs, pull=directed, nthreads=8), rtol=RTOL, atol=0)
+    for i in range(0, k, max(1, k // 8)):
+        _, _, ref = oracle.brandes(hg.R, hg.C, n, int(srcs[i]), "pull" if directed else "f64")
+        np.testing.assert_allclose(delta[i].cpu().numpy(), ref, rtol=RTOL, atol=0)
+
+
+@pytest.mark.parametrize("n,m,k", [(2, 1, 2), (7, 12, 7), (33, 300, 33), (64, 2000, 64), (1023, 8000, 200), (1025, 30000, 700),
+                                   (4097, 150000, 40), (8191, 40000, 300), (8192, 400000, 20)])
+@pytest.mark.parametrize("directed", [False, True])
+def test_sizes(n, m, k, directed):
+    rng = np.random.default_rng(n + directed)
+    u, v = rng.integers(0, n, m), rng.integers(0, n, m)
+    if n > 1000:  # hubs: lists of a few entries up to thousands in one level
+        hub = rng.integers(0, n, 3)
+        u = np.concatenate([u, np.repeat(hub, 700)])
+        v = np.concatenate([v, rng.integers(0, n, 2100)])
+    hg = gu.HostGraph.from_edges(n, u, v, symmetric=not directed)
+    check(hg, gu.sources(n, k, seed=3), directed)
+
+
+def test_shapes():
+    path = gu.HostGraph.from_edges(900, np.arange(899), np.arange(1, 900))  # 900 levels of one vertex
+    check(path, np.array([0, 450, 899], np.int32))
+    star = gu.HostGraph.from_edges(8000, np.zeros(7990, np.int32), np.arange(1, 7991))  # one list of 7990, isolated ends
+    check(star, np.array([0, 5, 7999, 5], np.int32))
+    # complete bipartite layers: lists of 63, 64 and 65 successors at every level
+    for w in (32, 63, 64, 65):
+        a, b = np.meshgrid(np.arange(w), np.arange(w))
+        u = np.concatenate([(l * w + a).ravel() for l in range(5)])
+        v = np.concatenate([((l + 1) * w + b).ravel() for l in range(5)])
+        check(gu.HostGraph.from_edges(6 * w, u, v), np.arange(0, 6 * w, 11, dtype=np.int32))
+
+
+def test_counts_wrap_and_wide_ranges():
+    """8-wide complete layers: 8^(l - 1) paths to level l, past 2^64 (the counts wrap, as
+    the oracle's do); with 12 layers the successors' terms span 2^33 and the
+    dependencies still agree."""
+    a, b = np.meshgrid(np.arange(8), np.arange(8))
+    for layers in (30, 12):
+        u = np.concatenate([(l * 8 + a).ravel() for l in range(layers - 1)] + [np.full(8, 8 * layers - 1), [0]])
+        v = np.concatenate([((l + 1) * 8 + b).ravel() for l in range(layers - 1)] + [np.arange(8) + 8 * layers, [8 * layers]])
+        hg = gu.HostGraph.from_edges(8 * layers + 8, u, v)
+        if layers == 12:
+            check(hg, np.arange(0, hg.n, 5, dtype=np.int32))
+            continue
+        g = gu.Graph(hg)
+        s = torch.tensor([0, 3, 100], dtype=torch.int32, device="cuda")
+        sig = torch.empty((3, hg.n), dtype=torch.int64, device="cuda")
+        g.sigma(s, sig)
+        _, rs = oracle.sigma_multi(hg.R, hg.C, hg.n, np.array([0, 3, 100], np.int32))
+        np.testing.assert_array_equal(sig.cpu().numpy().view(np.uint64), rs)
+
+
+def test_bad_sources_and_batches():
+    hg = gu.HostGraph.rmat(9, 8, seed=1)
+    g = gu.Graph(hg)
+    bc = torch.full((hg.n,), -7.0, dtype=torch.float64, device="cuda")
+    sig = torch.empty((2, hg.n), dtype=torch.int64, device="cuda")
+    for bad in (hg.n, -1):
+        s = torch.tensor([0, bad], dtype=torch.int32, device="cuda")
+        for call in (lambda: g.bc(s, bc), lambda: g.sigma(s, sig)):
+            with pytest.raises(gu.GuError) as e:
+                call()
+            assert e.value.status == 1
+        assert (bc == -7.0).all()
+    s = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    for batch in (100, 192):
+        with pytest.raises(gu.GuError) as e:
+            g.bc(s, bc, batch=batch)
+        assert e.value.status == 1
+    srcs = gu.sources(hg.n, 200, seed=2)
+    s = torch.as_tensor(srcs, device="cuda")
+    ref = oracle.bc(hg.R, hg.C, hg.n, srcs, nthreads=4)
+    for batch in (0, 64, 256):  # 64: passes, the batched engine
+        g.bc(s, bc, batch=batch)
+        assert (g.level_profile() == []) == (batch != 64)
+        np.testing.assert_allclose(bc.cpu().numpy(), ref, rtol=RTOL, atol=0)
