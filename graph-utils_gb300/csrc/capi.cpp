@@ -1023,7 +1023,10 @@ gu_status gu_reach(gu_graph g, const int32_t *sources_dev, int32_t k, int64_t *c
         check_sources_device(dg, sources_dev, k, st);
         if (k == 0) return;
         auto *cnt = reinterpret_cast<unsigned long long *>(counts_dev);
+        const bool by_levels = dag_reach_first(dg, k);
+        if (by_levels && launch_dag_reach(dg, sources_dev, k, cnt, st)) return;
         if (launch_smem_bfs(dg, sources_dev, k, nullptr, dg.n, cnt, nullptr, st)) return;
+        if (!by_levels && launch_dag_reach(dg, sources_dev, k, cnt, st)) return;
         GU_CUDA_CHECK(cudaMemsetAsync(counts_dev, 0, sizeof(int64_t) * (size_t)k, st));
         if (auto_engine(dg) == AutoEngine::LOCAL &&
             launch_local_bfs(dg, sources_dev, k, nullptr, dg.n, cnt, nullptr, st))

@@ -25,6 +25,11 @@ constexpr int TOPO_THREADS = 512;
 constexpr int TOPO_MIN_BLOCKS = 3;
 constexpr int64_t TOPO_MAX_N = (int64_t)1 << 26;  // positions fit the packed append counter
 constexpr int CLOSURE_CHUNK = 4096;               // columns per warp step: 16 bytes per lane
+// Reachable counts by levels of the order: up to this many levels (about 3.5 us each;
+// a search takes about 10 us a level of its own, of which it may have far fewer), and
+// lists short enough for eight lanes.
+constexpr int REACH_MAX_LEVELS = 96;
+constexpr int32_t REACH_MAX_IN_DEGREE = 2048;
 // Rows kept at once: the closure runs in column blocks of at most this many bytes
 // of rows (n = 65536 fits one block; a block costs one pass over the levels, about
 // 3 us each, so narrower blocks that would stay in L2 cost more than they save).
@@ -38,6 +43,9 @@ struct TopoCtl {
     int pad[4];
     int nlevels, total;
     u64 pack[4];  // appended vertices of a level, (count << 38) | out-edges
+    u64 ins[4];   // ... and their in-edges
+    int top;      // reach_kernel: highest level of the batch's sources, plus one
+    int pad2;
 };
 constexpr int TOPO_PACK = 38;
 
@@ -49,36 +57,48 @@ struct TopoArgs {
     int32_t n;
     int64_t m;
     int32_t *cnt;  // successors not yet placed
-    int32_t *pos;  // position of a vertex
-    int32_t *order, *lvl, *PR, *PC;
+    int2 *in;      // in-list ends (RT) by position
+    int32_t *pos;  // position of a vertex (kept)
+    int32_t *order, *lvl, *PR, *PC, *IC;
+    int2 *IR;
     TopoCtl *ctl;
     unsigned long long wait_ns;
 };
 
-// All lanes of the warp call it; lanes with pred place their vertex at the end of
-// the level being collected (one 64-bit atomic per warp reserves the positions and
-// the out-edge range).
-__device__ __forceinline__ void topo_place(const TopoArgs &a, u64 *pack, long long base_p, long long base_e, bool pred,
-                                           int32_t v)
+// All lanes of the warp call it; lanes with pred place their vertex (out-degree deg,
+// in-list ends in) at the end of the level being collected: one 64-bit atomic per warp
+// reserves the positions and the out-edge range, another, by a second lane at once, the
+// in-edge range.  (In-edge ranges are then not in position order: both ends are kept.)
+__device__ __forceinline__ void topo_place(const TopoArgs &a, int slot, long long base_p, long long base_e, long long base_i,
+                                           bool pred, int32_t v, unsigned deg, int2 in)
 {
     const unsigned mask = __ballot_sync(FULL_MASK, pred);
     if (!mask) return;
     const int lane = lane_id();
-    const unsigned deg = pred ? (unsigned)(__ldg(a.R + v + 1) - __ldg(a.R + v)) : 0u;
-    unsigned long long inc = deg;
+    const unsigned ind = pred ? (unsigned)(in.y - in.x) : 0u;
+    if (!pred) deg = 0;
+    unsigned inc = deg, inci = ind;  // (sums over distinct vertices: at most m)
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(FULL_MASK, inc, o);
-        if (lane >= o) inc += y;
+        const unsigned y = __shfl_up_sync(FULL_MASK, inc, o), z = __shfl_up_sync(FULL_MASK, inci, o);
+        if (lane >= o) {
+            inc += y;
+            inci += z;
+        }
     }
-    u64 old = 0;
-    if (lane == 31) old = atomicAdd(pack, ((u64)__popc(mask) << TOPO_PACK) | inc);
-    old = __shfl_sync(FULL_MASK, old, 31);
+    const unsigned toti = __shfl_sync(FULL_MASK, inci, 31);
+    u64 r = 0;
+    if (lane == 31) r = atomicAdd(&a.ctl->pack[slot], ((u64)__popc(mask) << TOPO_PACK) | inc);
+    if (lane == 30) r = atomicAdd(&a.ctl->ins[slot], (u64)toti);
+    const u64 old = __shfl_sync(FULL_MASK, r, 31), oldi = __shfl_sync(FULL_MASK, r, 30);
     if (pred) {
         const int32_t p = (int32_t)(base_p + (long long)(old >> TOPO_PACK) + __popc(mask & ((1u << lane) - 1u)));
         a.order[p] = v;
         a.pos[v] = p;
         a.PR[p] = (int32_t)(base_e + (long long)(old & ((1ull << TOPO_PACK) - 1ull)) + (long long)(inc - deg));
+        const int32_t i0 = (int32_t)(base_i + (long long)oldi + (long long)(inci - ind));
+        a.IR[p] = make_int2(i0, i0 + (int32_t)ind);
+        a.in[p] = in;
     }
 }
 
@@ -88,50 +108,61 @@ __device__ __forceinline__ void topo_place(const TopoArgs &a, u64 *pack, long lo
 // result does.
 __global__ void __launch_bounds__(TOPO_THREADS, TOPO_MIN_BLOCKS) topo_plan_kernel(TopoArgs a)
 {
-    __shared__ u64 s_pack[4];
+    __shared__ u64 s_pack[8];  // pack and ins
     unsigned epoch = 0;
     TopoCtl *ctl = a.ctl;
-    auto barrier = [&] { return grid_barrier(&ctl->bar, &ctl->err, epoch, a.wait_ns, ctl->pack, s_pack, 4); };
+    auto barrier = [&] { return grid_barrier(&ctl->bar, &ctl->err, epoch, a.wait_ns, ctl->pack, s_pack, 8); };
     const long long rank = (long long)blockIdx.x * blockDim.x + threadIdx.x, size = (long long)gridDim.x * blockDim.x;
-    const long long gw = rank >> 5, nw = size >> 5;
-    const int lane = lane_id();
-    for (long long b = gw * 32; b < a.n; b += nw * 32) {  // warp-uniform
-        const long long v = b + lane;
+    const long long ngrp = size >> 3;
+    const int sub = lane_id() & 7;
+    for (long long b = rank & ~31ll; b < a.n; b += size) {  // warp-uniform
+        const long long v = b + lane_id();
         int32_t d = 1;
+        int2 in = make_int2(0, 0);
         if (v < a.n) {
             d = __ldg(a.R + v + 1) - __ldg(a.R + v);
+            in = make_int2(__ldg(a.RT + v), __ldg(a.RT + v + 1));
             a.cnt[v] = d;
         }
-        topo_place(a, &ctl->pack[0], 0, 0, d == 0, (int32_t)v);
+        topo_place(a, 0, 0, 0, 0, d == 0, (int32_t)v, 0, in);
     }
     if (!barrier()) return;
-    long long ls = 0, ebase = 0;
+    long long ls = 0, ebase = 0, ibase = 0;
     int level = 0;
     for (;; ++level) {
         const u64 pk = s_pack[level & 3];
         const long long le = ls + (long long)(pk >> TOPO_PACK);
         if (le == ls) break;
         const long long enext = ebase + (long long)(pk & ((1ull << TOPO_PACK) - 1ull));
+        const long long inext = ibase + (long long)s_pack[4 + (level & 3)];
         if (rank == 0) {
             a.lvl[level] = (int32_t)ls;
+            ctl->ins[(level + 2) & 3] = 0;
             ctl->pack[(level + 2) & 3] = 0;  // collects level + 2; last read two levels ago
         }
-        for (long long p = ls + gw; p < le; p += nw) {
-            const int32_t v = __ldcg(a.order + p);
-            const int32_t e1 = __ldg(a.RT + v + 1);
-            for (int32_t eb = __ldg(a.RT + v); eb < e1; eb += 32) {
+        // eight lanes per vertex of the level, their in-lists' ends kept when it was placed
+        for (long long p0 = ls + (rank >> 5) * 4; p0 < le; p0 += ngrp) {  // warp-uniform
+            const long long p = p0 + (lane_id() >> 3);
+            const int2 r = p < le ? __ldcg(a.in + p) : make_int2(0, 0);
+            for (int32_t e = r.x + sub; __any_sync(FULL_MASK, e < r.y); e += 8) {
                 int32_t u = 0;
                 bool last = false;
-                if (eb + lane < e1) {
-                    u = __ldg(a.CT + eb + lane);
+                int2 in = make_int2(0, 0);
+                unsigned d = 0;
+                if (e < r.y) {
+                    u = __ldg(a.CT + e);
+                    // (the degrees in case it is placed, with the decrement and not after it)
+                    d = (unsigned)(__ldg(a.R + u + 1) - __ldg(a.R + u));
+                    in = make_int2(__ldg(a.RT + u), __ldg(a.RT + u + 1));
                     last = atomicSub(a.cnt + u, 1) == 1;
                 }
-                topo_place(a, &ctl->pack[(level + 1) & 3], le, enext, last, u);
+                topo_place(a, (level + 1) & 3, le, enext, inext, last, u, d, in);
             }
         }
         if (!barrier()) return;
         ls = le;
         ebase = enext;
+        ibase = inext;
     }
     if (rank == 0) {
         a.lvl[level] = (int32_t)ls;
@@ -140,12 +171,14 @@ __global__ void __launch_bounds__(TOPO_THREADS, TOPO_MIN_BLOCKS) topo_plan_kerne
     }
     if (ls != a.n) return;
     if (rank == 0) a.PR[a.n] = (int32_t)a.m;
-    // successors in position space, eight lanes per vertex
-    const int sub = lane & 7;
+    // neighbours in position space, eight lanes per vertex
     for (long long p = rank >> 3; p < a.n; p += size >> 3) {
         const int32_t v = __ldcg(a.order + p);
         const int32_t e0 = __ldg(a.R + v), d = __ldg(a.R + v + 1) - e0, o = __ldcg(a.PR + p);
         for (int32_t i = sub; i < d; i += 8) a.PC[o + i] = __ldcg(a.pos + __ldg(a.C + e0 + i));
+        const int32_t f0 = __ldg(a.RT + v);
+        const int2 r = __ldcg(a.IR + p);
+        for (int32_t i = sub; i < r.y - r.x; i += 8) a.IC[r.x + i] = __ldcg(a.pos + __ldg(a.CT + f0 + i));
     }
 }
 
@@ -232,6 +265,180 @@ __global__ void __launch_bounds__(TOPO_THREADS, TOPO_MIN_BLOCKS) closure_kernel(
     }
 }
 
+// ---- reachable counts of k sources -------------------------------------------------
+struct ReachArgs {
+    const int32_t *__restrict__ pos;
+    const int32_t *__restrict__ lvl;
+    const int2 *__restrict__ IR;
+    const int32_t *__restrict__ IC;
+    int32_t n, nlevels;
+    const int32_t *__restrict__ sources;
+    int32_t k;
+    u64 *rows;  // [n][W] by position: the sources that reach the vertex
+    unsigned long long *counts;
+    TopoCtl *ctl;
+    unsigned long long wait_ns;
+};
+
+// Vertices reached by each source of the batch: a thread adds up to 15 of the rows'
+// words in bit slices (four 64-bit planes: a count of four bits for each of 64
+// sources), the lanes that hold the same word add their slices, and each lane then
+// reads its share of the sources' counts.
+template <int W>
+__device__ void count_rows(const u64 *rows, size_t words, unsigned *s_cnt, long long rank, long long size)
+{
+    constexpr int PER = 2 * W;  // sources per lane: 64 among the 32 / W lanes of a word
+    constexpr int PLANES = W == 1 ? 9 : W == 2 ? 8 : 7;  // 15 words x 32 / W lanes
+    const int lane = lane_id();
+    unsigned sum[PER] = {};
+    for (size_t i0 = 0; i0 < words; i0 += 15 * (size_t)size) {  // warp-uniform
+        u64 c[PLANES] = {};
+#pragma unroll 5
+        for (int j = 0; j < 15; ++j) {
+            const size_t i = i0 + (size_t)j * size + rank;
+            u64 x = i < words ? __ldcg(rows + i) : 0ull;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const u64 y = c[b] & x;
+                c[b] ^= x;
+                x = y;
+            }
+        }
+#pragma unroll
+        for (int r = 0, o = W; o < 32; ++r, o <<= 1) {
+            u64 carry = 0;
+#pragma unroll
+            for (int b = 0; b < PLANES; ++b) {
+                if (b > 4 + r) break;
+                const u64 y = __shfl_xor_sync(FULL_MASK, c[b], o), z = c[b] ^ y;
+                const u64 s = z ^ carry;
+                carry = (c[b] & y) | (z & carry);
+                c[b] = s;
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < PER; ++s) {
+            const int bit = (lane / W) * PER + s;
+#pragma unroll
+            for (int b = 0; b < PLANES; ++b) sum[s] += (unsigned)((c[b] >> bit) & 1ull) << b;
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < PER; ++s)
+        if (sum[s]) atomicAdd(s_cnt + 64 * (lane % W) + (lane / W) * PER + s, sum[s]);
+}
+
+// Levels from the highest source's down: a vertex's row is its own sources' bits and
+// the OR of its predecessors' rows, eight lanes per vertex, one grid barrier per level.
+// Every vertex is visited once, where the level-synchronous search expands it at each
+// distance at which a source first meets it.  The next level's lists are asked for
+// before the barrier, so that only the rows are waited for after it.  Bound: the levels'
+// chain (rows, barrier), about 2.7 us each.  DAG of 200,003 vertices, m = 8 n, 200
+// sources: 151 us (0.19 ms a call), the search 377 us (0.42 ms).
+template <int W>
+__global__ void __launch_bounds__(TOPO_THREADS, 2) reach_kernel(ReachArgs a)
+{
+    __shared__ unsigned s_cnt[64 * W];
+    __shared__ int s_top;
+    unsigned epoch = 0;
+    TopoCtl *ctl = a.ctl;
+    auto barrier = [&] { return grid_barrier(&ctl->bar, &ctl->err, epoch, a.wait_ns); };
+    const long long rank = (long long)blockIdx.x * blockDim.x + threadIdx.x, size = (long long)gridDim.x * blockDim.x;
+    const long long grp = rank >> 3, ngrp = size >> 3;
+    const int sub = threadIdx.x & 7;
+    const size_t words = (size_t)a.n * W;
+    for (int32_t row0 = 0; row0 < a.k; row0 += 64 * W) {
+        const int nb = min(64 * W, a.k - row0);
+        for (size_t i = (size_t)rank; i < words; i += (size_t)size) a.rows[i] = 0ull;
+        if (rank == 0) ctl->top = 0;
+        if (!barrier()) return;
+        if (rank < nb) {
+            const int32_t p = __ldg(a.pos + __ldg(a.sources + row0 + rank));
+            atomicOr(a.rows + (size_t)p * W + (rank >> 6), 1ull << (rank & 63));
+            int lo = 0, hi = a.nlevels - 1;  // the level of position p
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(a.lvl + mid) <= p) lo = mid;
+                else hi = mid - 1;
+            }
+            atomicMax(&ctl->top, lo);
+        }
+        if (!barrier()) return;
+        if (threadIdx.x == 0) s_top = ld_volatile_i32(&ctl->top);
+        __syncthreads();
+        // this group's first vertex of a level: its list's ends and this lane's first entry
+        int32_t ls = 0, le = 0, e = 0, e1 = 0, q = 0;
+        auto first = [&](int l) {
+            ls = __ldg(a.lvl + l);
+            le = __ldg(a.lvl + l + 1);
+            e = e1 = 0;
+            if (ls + grp < le) {
+                const int2 r = __ldg(a.IR + ls + grp);
+                e = r.x + sub;
+                e1 = r.y;
+                if (e < e1) q = __ldg(a.IC + e);
+            }
+        };
+        if (s_top > 0) first(s_top - 1);
+        for (int l = s_top - 1; l >= 0; --l) {
+            for (long long p = ls + grp; __any_sync(FULL_MASK, p < le); p += ngrp) {  // warp-uniform trips
+                if (p != ls + grp) {
+                    e = e1 = 0;
+                    if (p < le) {
+                        const int2 r = __ldg(a.IR + p);
+                        e = r.x + sub;
+                        e1 = r.y;
+                        if (e < e1) q = __ldg(a.IC + e);
+                    }
+                }
+                u64 acc[W] = {};
+                if (p < le && sub == 0) {  // its own sources
+#pragma unroll
+                    for (int w = 0; w < W; ++w) acc[w] = __ldcg(a.rows + (size_t)p * W + w);
+                }
+                while (e < e1) {
+                    const int32_t qn = e + 8 < e1 ? __ldg(a.IC + e + 8) : 0;
+                    const u64 *r = a.rows + (size_t)q * W;
+                    if constexpr (W == 4) {
+                        u64 x0, x1, x2, x3;
+                        asm volatile("ld.global.cg.v4.u64 {%0, %1, %2, %3}, [%4];"
+                                     : "=l"(x0), "=l"(x1), "=l"(x2), "=l"(x3) : "l"(r) : "memory");
+                        acc[0] |= x0, acc[1] |= x1, acc[2] |= x2, acc[3] |= x3;
+                    } else {
+#pragma unroll
+                        for (int w = 0; w < W; ++w) acc[w] |= __ldcg(r + w);
+                    }
+                    q = qn;
+                    e += 8;
+                }
+                u64 any = 0;
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) acc[w] |= __shfl_xor_sync(FULL_MASK, acc[w], o);
+                    any |= acc[w];
+                }
+                if (p < le && sub < W && any) {
+                    u64 mine = acc[0];
+#pragma unroll
+                    for (int w = 1; w < W; ++w)
+                        if (sub == w) mine = acc[w];
+                    a.rows[(size_t)p * W + sub] = mine;
+                }
+            }
+            if (l > 0) first(l - 1);  // static lists: loads in flight across the barrier
+            if (!barrier()) return;
+        }
+        for (int i = threadIdx.x; i < 64 * W; i += blockDim.x) s_cnt[i] = 0;
+        __syncthreads();
+        count_rows<W>(a.rows, words, s_cnt, rank, size);
+        __syncthreads();
+        for (int i = threadIdx.x; i < nb; i += blockDim.x)
+            if (s_cnt[i]) atomicAdd(a.counts + row0 + i, (unsigned long long)s_cnt[i]);
+        if (row0 + 64 * W < a.k && !barrier()) return;  // the rows are cleared for the next batch
+    }
+}
+
 template <class K>
 static int topo_grid(K kern, int sms)
 {
@@ -248,14 +455,14 @@ static void check_topo(const TopoCtl &c)
 }
 
 // Builds the graph's topological order once (synchronises st); false if the graph
-// has a cycle.
-static bool ensure_topo(DeviceGraph &g, cudaStream_t st)
+// has a cycle.  ws_bytes: workspace that the caller takes next (allocated at once).
+static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
 {
     TopoPlan &t = g.topo;
     if (t.state != TopoPlan::UNBUILT) return t.state == TopoPlan::ACYCLIC;
     const size_t n = (size_t)g.n, m = (size_t)g.m;
-    char *ws = (char *)g.ws.get(WS_CONTROL_BYTES + 2 * n * sizeof(int32_t));
-    const size_t ints = n + (n + 2) + (n + 1) + m;
+    char *ws = (char *)g.ws.get(std::max(ws_bytes, WS_CONTROL_BYTES + 3 * n * sizeof(int32_t)));
+    const size_t ints = 2 * n + 2 * n + (n + 2) + (n + 1) + 2 * m;
     int32_t *buf = nullptr;
     const cudaError_t e = dev_malloc((void **)&buf, ints * sizeof(int32_t));
     if (e != cudaSuccess) {
@@ -271,26 +478,31 @@ static bool ensure_topo(DeviceGraph &g, cudaStream_t st)
     a.CT = g.CT;
     a.n = g.n;
     a.m = g.m;
-    a.cnt = reinterpret_cast<int32_t *>(ws + WS_CONTROL_BYTES);
-    a.pos = a.cnt + n;
-    a.order = buf;
-    a.lvl = buf + n;
+    a.in = reinterpret_cast<int2 *>(ws + WS_CONTROL_BYTES);
+    a.cnt = reinterpret_cast<int32_t *>(a.in + n);
+    a.IR = reinterpret_cast<int2 *>(buf);
+    a.order = buf + 2 * n;
+    a.pos = a.order + n;
+    a.lvl = a.pos + n;
     a.PR = a.lvl + n + 2;
     a.PC = a.PR + n + 1;
+    a.IC = a.PC + m;
     a.ctl = reinterpret_cast<TopoCtl *>(ws);
     a.wait_ns = wait_limit_ns();
     GU_CUDA_CHECK(cudaMemsetAsync(ws, 0, WS_CONTROL_BYTES, st));
     void *params[] = {&a};
-    GU_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)topo_plan_kernel, dim3(topo_grid(topo_plan_kernel, g.sm_count)),
-                                              dim3(TOPO_THREADS), params, 0, st));
+    GU_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)topo_plan_kernel, dim3(g.sm_count), dim3(TOPO_THREADS), params, 0, st));
     TopoCtl c;
     GU_CUDA_CHECK(cudaMemcpyAsync(&c, ws, sizeof(c), cudaMemcpyDeviceToHost, st));
     GU_CUDA_CHECK(cudaStreamSynchronize(st));
     check_topo(c);
     t.order = a.order;
     t.lvl = a.lvl;
+    t.pos = a.pos;
     t.PR = a.PR;
     t.PC = a.PC;
+    t.IR = reinterpret_cast<int32_t *>(a.IR);
+    t.IC = a.IC;
     t.nlevels = c.nlevels;
     t.state = c.total == g.n ? TopoPlan::ACYCLIC : TopoPlan::CYCLIC;
     return t.state == TopoPlan::ACYCLIC;
@@ -306,13 +518,14 @@ static bool launch_closure(DeviceGraph &g, unsigned long long *counts, cudaStrea
     char *ws = nullptr;
     int64_t block = 0;
     try {
-        if (!ensure_topo(g, st)) return false;
         // equal column blocks within the row budget, at least one chunk wide
         const int64_t fit = std::max<int64_t>(1, (int64_t)(CLOSURE_ROWS_BYTES / (n * (CLOSURE_CHUNK / 8))));
         const int64_t chunks = ((int64_t)n + CLOSURE_CHUNK - 1) / CLOSURE_CHUNK;
         const int64_t nblocks = (chunks + fit - 1) / fit;
         block = (chunks + nblocks - 1) / nblocks * CLOSURE_CHUNK;
-        ws = (char *)g.ws.get(WS_CONTROL_BYTES + n * (size_t)(block / 8));
+        const size_t need = WS_CONTROL_BYTES + n * (size_t)(block / 8);
+        if (!ensure_topo(g, need, st)) return false;
+        ws = (char *)g.ws.get(need);
     } catch (const gu_error &e) {
         if (e.code == GU_ERR_OUT_OF_MEMORY) return false;
         throw;
@@ -336,6 +549,56 @@ static bool launch_closure(DeviceGraph &g, unsigned long long *counts, cudaStrea
     GU_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)closure_kernel, dim3(topo_grid(closure_kernel, g.sm_count)),
                                               dim3(TOPO_THREADS), params, 0, st));
     g.mark_stop(st);
+    return true;
+}
+
+// Reachable counts of k sources (themselves included) on an acyclic graph; false where
+// this does not apply.  Synchronises st.
+bool launch_dag_reach(DeviceGraph &g, const int32_t *sources, int32_t k, unsigned long long *counts, cudaStream_t st)
+{
+    const char *env = std::getenv("GU_AUTO_LOCAL");
+    if (env && env[0] == '0') return false;
+    if (!g.directed || g.n < 1 || g.n > TOPO_MAX_N || g.max_in_degree > REACH_MAX_IN_DEGREE) return false;
+    char *ws = nullptr;
+    const int W = msbfs_words_for(k);
+    // The order costs about as much to build as the searches that it replaces save in one
+    // call (n = 200,003: 0.55 ms; 0.42 -> 0.19 ms a call): a graph that is asked once is
+    // searched, and the order is built when it is asked again.
+    if (g.topo.state == TopoPlan::UNBUILT && g.topo.asked++ == 0) return false;
+    try {
+        const size_t need = WS_CONTROL_BYTES + sizeof(u64) * (size_t)g.n * W;
+        if (!ensure_topo(g, need, st) || g.topo.nlevels > REACH_MAX_LEVELS) return false;
+        ws = (char *)g.ws.get(need);
+    } catch (const gu_error &e) {
+        if (e.code == GU_ERR_OUT_OF_MEMORY) return false;
+        throw;
+    }
+    ReachArgs a;
+    a.pos = g.topo.pos;
+    a.lvl = g.topo.lvl;
+    a.IR = reinterpret_cast<const int2 *>(g.topo.IR);
+    a.IC = g.topo.IC;
+    a.n = g.n;
+    a.nlevels = g.topo.nlevels;
+    a.sources = sources;
+    a.k = k;
+    a.rows = reinterpret_cast<u64 *>(ws + WS_CONTROL_BYTES);
+    a.counts = counts;
+    a.ctl = reinterpret_cast<TopoCtl *>(ws);
+    a.wait_ns = wait_limit_ns();
+    GU_CUDA_CHECK(cudaMemsetAsync(ws, 0, WS_CONTROL_BYTES, st));
+    GU_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int64_t) * (size_t)k, st));
+    g.timeline = 0;
+    g.mark_start(st);
+    const void *kern = W == 1 ? (const void *)reach_kernel<1> : W == 2 ? (const void *)reach_kernel<2> : (const void *)reach_kernel<4>;
+    void *params[] = {&a};
+    // one CTA per SM: a level's vertices seldom need more groups, and the barrier is cheaper
+    GU_CUDA_CHECK(cudaLaunchCooperativeKernel(kern, dim3(g.sm_count), dim3(TOPO_THREADS), params, 0, st));
+    g.mark_stop(st);
+    TopoCtl c = {};
+    GU_CUDA_CHECK(cudaMemcpyAsync(&c, ws, sizeof(c), cudaMemcpyDeviceToHost, st));
+    GU_CUDA_CHECK(cudaStreamSynchronize(st));
+    check_topo(c);
     return true;
 }
 

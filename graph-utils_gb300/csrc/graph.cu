@@ -297,6 +297,7 @@ DeviceGraph *create_device_graph(const int32_t *R, const int32_t *C, int32_t n, 
             for (int32_t v = 0; v < n; ++v) indeg[v] = R[v + 1] - R[v];
         }
         for (int32_t v = 0; v < n; ++v) {
+            if (indeg[v] > g->max_in_degree) g->max_in_degree = indeg[v];
             if (indeg[v] > BU_HEAVY_DEGREE) heavy.push_back(v);
             else if (indeg[v] > BU_MID_DEGREE) wide.push_back(v);
             else if (indeg[v] > BU_LIGHT_DEGREE) mid.push_back(v);

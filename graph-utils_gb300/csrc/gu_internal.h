@@ -146,7 +146,11 @@ struct TopoPlan {
     int32_t *lvl = nullptr;    // [nlevels + 1] first position of each level
     int32_t *PR = nullptr;     // [n + 1] out-edge offsets by position
     int32_t *PC = nullptr;     // [m] positions of the successors
+    int32_t *pos = nullptr;    // [n] position of a vertex
+    int32_t *IR = nullptr;     // [n][2] first and end in-edge by position
+    int32_t *IC = nullptr;     // [m] positions of the predecessors
     int nlevels = 0;
+    int asked = 0;             // reachability calls that came before it was built
 };
 
 struct DeviceGraph {
@@ -157,7 +161,7 @@ struct DeviceGraph {
     int32_t *R = nullptr, *C = nullptr;
     int32_t *RT = nullptr, *CT = nullptr;
     int32_t *F = nullptr;
-    int32_t max_degree = 0;
+    int32_t max_degree = 0, max_in_degree = 0;
     // AUTO's measured choice (gu_graph_autotune / gu_graph_set_tuning); unset: by shape
     struct Tuning {
         bool set = false;
@@ -244,6 +248,12 @@ void launch_plain_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
 // if a frontier overflowed its shared queues (rerun on the batched engine).
 // Reachable-set sizes of every vertex of a DAG (self excluded) and their sum.
 void dag_reach(DeviceGraph &g, int64_t *counts, int64_t *total_host, cudaStream_t st);
+// ... and whether it goes before the shared-memory engine, where both apply: above the
+// sizes that engine takes whole, for more than a few sources (call times, this form /
+// that engine: DAG of 60000 vertices k = 1 100 / 37 us, k = 100 180 / 451; 5000 vertices
+// k = 100 140 / 78).
+inline bool dag_reach_first(const DeviceGraph &g, int32_t k) { return g.directed && g.n > 16384 && k > 4; }
+bool launch_dag_reach(DeviceGraph &g, const int32_t *sources, int32_t k, unsigned long long *counts, cudaStream_t st);
 int msbfs_words_for(int32_t k);  // 64-source words per batch for k sources
 enum class AutoEngine { LOCAL, BATCHED };
 AutoEngine auto_engine(const DeviceGraph &g);

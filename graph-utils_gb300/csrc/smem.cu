@@ -655,10 +655,11 @@ static SbConfig sb_config(const DeviceGraph &g, int S, int threads)
 //   n <= 32768: up to one source per SM and k m = 140 M (R-MAT 15 k = 150 90 / 174,
 //     ER 30000 k = 150 98 / 143; k = 300 196 / 254, but behind on denser graphs).
 //   above, by k m, the work that the batched engine shares among the sources: up to
-//     60 M (R-MAT 16 k = 32 70 / 143, ER 65000 k = 40 134 / 133, ER 100000 k = 30
-//     131 / 143; ER 65000 k = 80 226 / 157), and beyond 131072 vertices, where a
-//     source needs eight CTAs, up to 8 sources (R-MAT 18 k = 8 115 / 153, k = 16
-//     179 / 167).
+//     60 M (R-MAT 16 k = 32 70 / 143, ER 100000 k = 30 131 / 143; ER 65000 k = 80 226 /
+//     157), with four CTAs a source at least (a DAG of 60000 vertices and 26 levels,
+//     counts, k = 100, one CTA a source: 451 / 305), and beyond 131072 vertices, where
+//     a source needs eight CTAs, up to 8 sources (R-MAT 18 k = 8 115 / 153, k = 16 179 /
+//     167).
 // Cluster size: as many CTAs per source as all k keep resident at once, while a CTA
 // has at least 4096 vertices (R-MAT 17 k = 1: S = 4 83 us, 8 65, 16 58; R-MAT 14
 // k = 1: S = 1 47, 4 43, 16 43).
@@ -679,11 +680,12 @@ static SbConfig sb_choose(const DeviceGraph &g, int32_t k)
         return SbConfig();
     }
     if (g.n >= 16384 && !low)
-        for (int S = SB_MAX_CLUSTER; S > 1; S /= 2) {
+        for (int S = SB_MAX_CLUSTER; S > (g.n > 32768 ? 2 : 1); S /= 2) {
             if (g.n / S < 4096) continue;
             const SbConfig c = sb_config(g, S, g.n / S <= (S == SB_MAX_CLUSTER ? 4096 : 8192) ? 512 : 1024);
             if (c.resident >= k) return c;
         }
+    if (g.n > 32768) return SbConfig();
     const int threads = g.n <= 4096 ? (many ? 256 : 512) : g.n <= 16384 ? (many || low ? 512 : 1024) : 1024;
     SbConfig c = sb_config(g, 1, threads);
     return c.resident > 0 ? c : SbConfig();

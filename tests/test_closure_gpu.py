@@ -76,3 +76,51 @@ def test_no_memory_for_rows_falls_back():
     np.testing.assert_array_equal(cnt.cpu().numpy(), ref)
     assert g.dag_reach(cnt) == rtot
     np.testing.assert_array_equal(cnt.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("n,m,k", [(16385, 60000, 5), (17001, 90000, 64), (20011, 100000, 65), (30000, 120000, 128),
+                                   (40000, 300000, 129), (70001, 280000, 256), (50000, 50000, 600)])
+def test_reach_by_levels_vs_search(n, m, k, monkeypatch):
+    """gu_reach on an acyclic graph (rows of source bits, level by level): counts equal
+    the oracle's and the batched search's at every row width and across batches, with
+    duplicate and sink sources."""
+    rng = np.random.default_rng(n)
+    a, b = rng.integers(0, n, m), rng.integers(0, n, m)
+    keep = a != b
+    perm = rng.permutation(n)
+    hub = perm[n - 1]  # one vertex with a long in-list
+    u = np.concatenate([perm[np.minimum(a, b)[keep]], perm[:1500]])
+    v = np.concatenate([perm[np.maximum(a, b)[keep]], np.full(1500, hub)])
+    hg = gu.HostGraph.from_edges(n, u, v, symmetric=False)
+    g = gu.Graph(hg)
+    srcs = gu.sources(n, k, seed=4)
+    srcs[:3] = [perm[n - 1], perm[0], perm[0]]
+    s = torch.as_tensor(srcs, device="cuda")
+    cnt = torch.full((k,), -1, dtype=torch.int64, device="cuda")
+    g.reach(s, cnt)  # the first call searches, the next ones have the order
+    first = cnt.cpu().numpy()
+    for _ in range(2):
+        cnt.fill_(-1)
+        g.reach(s, cnt)
+        np.testing.assert_array_equal(cnt.cpu().numpy(), first)
+    assert g.level_profile() == []  # no search ran
+    got = cnt.cpu().numpy()
+    monkeypatch.setenv("GU_AUTO_LOCAL", "0")
+    g.reach(s, cnt)
+    np.testing.assert_array_equal(got, cnt.cpu().numpy())
+    some = list(range(0, k, max(1, k // 6)))
+    ref, _ = oracle.bfs_multi(hg.R, hg.C, n, srcs[some], nthreads=8)
+    np.testing.assert_array_equal(got[some], (ref != gu.UNREACHABLE).sum(1))
+
+
+def test_reach_on_deep_and_cyclic_graphs():
+    n = 20000
+    chain = gu.HostGraph.from_edges(n, np.arange(n - 1), np.arange(1, n), symmetric=False)  # too many levels
+    ring = gu.HostGraph.from_edges(n, np.arange(n), (np.arange(n) + 1) % n, symmetric=False)  # a cycle
+    s = torch.arange(0, n, 2500, dtype=torch.int32, device="cuda")
+    for hg, want in ((chain, n - np.arange(0, n, 2500)), (ring, np.full(8, n))):
+        g = gu.Graph(hg)
+        for _ in range(3):
+            cnt = torch.full((8,), -1, dtype=torch.int64, device="cuda")
+            g.reach(s, cnt)
+            np.testing.assert_array_equal(cnt.cpu().numpy(), want)
