@@ -288,9 +288,15 @@ struct MsQueueRequest {
     unsigned long long *reach = nullptr;
 };
 struct MsQueueLaunch {
-    int W = 0, ngroups = 0, group_size = 0, items = 0;
-    size_t stride = 0;                             // bytes of workspace per group
-    size_t items_off = 0, cnt_off = 0, bytes = 0;  // item array, counter, total workspace
+    struct Group {
+        int base, size;  // CTAs
+        int first;       // its first item, -1: from the counter
+        size_t data;     // its workspace slice
+    };
+    int W = 0, items = 0, grid = 0;
+    int taken = 0;  // items given out as the groups' first ones: where the counter starts
+    std::vector<Group> groups;
+    size_t items_off = 0, groups_off = 0, cnt_off = 0, bytes = 0;  // workspace: items, groups, counter, total
 };
 MsQueueLaunch msbfs_queue_plan(const std::vector<MsQueueRequest> &reqs, int sms, int max_blocks);
 // Runs every request in one persistent launch whose CTA groups drain a device

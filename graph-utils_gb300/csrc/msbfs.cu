@@ -47,6 +47,7 @@
 #include <climits>
 #include <cstddef>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 namespace gu {
@@ -1773,19 +1774,19 @@ __host__ __device__ inline int ms_planes(size_t n)
     while (nplanes < MAX_PLANES && ((int64_t)(n > 0 ? n - 1 : 0) >> nplanes) != 0) ++nplanes;
     return nplanes;
 }
-__host__ __device__ inline size_t ms_layout_bytes(size_t n, int W)
+__host__ __device__ inline size_t ms_data_bytes(size_t n, int W)
 {
-    return WS_CONTROL_BYTES + (4 + (size_t)ms_planes(n)) * ms_up256(n * W * sizeof(u64)) +
+    return (4 + (size_t)ms_planes(n)) * ms_up256(n * W * sizeof(u64)) +
            7 * ms_up256(n * sizeof(int32_t));
 }
-__host__ __device__ inline void ms_layout(char *ws, size_t n, int W, MsArgs &a)
+__host__ __device__ inline size_t ms_layout_bytes(size_t n, int W) { return WS_CONTROL_BYTES + ms_data_bytes(n, W); }
+// control region at ctl, the arrays from p on (256-byte aligned)
+__host__ __device__ inline void ms_layout(char *ctl, char *p, size_t n, int W, MsArgs &a)
 {
     const size_t words_bytes = ms_up256(n * W * sizeof(u64));
     const size_t i32_bytes = ms_up256(n * sizeof(int32_t));
-    char *p = ws;
-    a.ctl = reinterpret_cast<MsCtl *>(p);
-    a.cover = reinterpret_cast<int *>(p + COVER_OFF);
-    p += WS_CONTROL_BYTES;
+    a.ctl = reinterpret_cast<MsCtl *>(ctl);
+    a.cover = reinterpret_cast<int *>(ctl + COVER_OFF);
     a.seen = reinterpret_cast<u64 *>(p);
     p += words_bytes;
     for (int i = 0; i < 3; ++i) {
@@ -1806,12 +1807,19 @@ __host__ __device__ inline void ms_layout(char *ws, size_t n, int W, MsArgs &a)
 }
 
 // ---- work-queue launch: many graphs and source blocks in one persistent grid ----
-// The grid is cut into groups of group_size consecutive CTAs.  A group's first CTA
-// takes the next item from a device counter and the group barrier hands it to the
-// group's other CTAs; the group then runs the batched search of that item (one
-// graph, up to 64 W sources) in its own slice of the workspace, with barriers over
-// its own CTAs only, and takes the next item until none is left.  Items of
-// different graphs and sizes run side by side on different groups.
+// The grid is cut into groups of consecutive CTAs.  A group starts with an item of its
+// own, if it was given one; then its first CTA takes the next item from a device
+// counter and the group barrier hands it to the group's other CTAs.  The group runs
+// the batched search of an item (one graph, up to 64 W sources) in its own slice of
+// the workspace, with barriers over its own CTAs only.  Items of different graphs and
+// sizes run side by side on different groups.
+//
+// With fewer items than half the grid's CTAs every item has its own group, sized by the
+// item's estimated work (queue_weight): with equal groups the largest graphs' items
+// bounded the launch while the small ones' groups stood idle (24 requests on R-MAT
+// 12-16 and DAGs of 65536 vertices: 1415 us, sized
+// 900 us).  With more items the
+// groups are equal and the counter balances them.
 struct MqItem {
     const int32_t *R, *C, *RT, *CT;
     const int32_t *light, *mid, *wide, *heavy;
@@ -1825,13 +1833,20 @@ struct MqItem {
     unsigned long long *reach;  // k reachable counts (zeroed before the launch), or null
 };
 
+struct MqGroup {
+    int base, nblk;   // its CTAs
+    int first;        // its first item (-1: from the counter)
+    int pad;
+    u64 data;         // offset of its workspace slice
+};
+
 struct MqArgs {
     const MqItem *items;
     int nitems;
-    int *next;           // item counter, zeroed before the launch
-    char *ws;            // group g's slice at ws + g * ws_stride
-    size_t ws_stride;
-    int group_size;
+    int *next;           // item counter, set before the launch
+    char *ws;            // group g's control region at ws + g * WS_CONTROL_BYTES
+    const MqGroup *groups;
+    int ngroups;
     float alpha, beta, gamma, rare_frac;
     unsigned long long wait_ns;
 };
@@ -1841,17 +1856,25 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) ms_queue_kernel(MqA
 {
     __shared__ int s_item;
     __shared__ MsArgs s_args;
-    const int grp = blockIdx.x / q.group_size;
+    __shared__ int s_grp;
     if (threadIdx.x == 0) {
-        s_grp_base = grp * q.group_size;
-        s_grp_nblk = min(q.group_size, (int)gridDim.x - grp * q.group_size);
+        int lo = 0, hi = q.ngroups - 1;  // the last group that starts at or before this CTA
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (q.groups[mid].base <= (int)blockIdx.x) lo = mid;
+            else hi = mid - 1;
+        }
+        s_grp = lo;
+        s_grp_base = q.groups[lo].base;
+        s_grp_nblk = q.groups[lo].nblk;
     }
     __syncthreads();
-    char *ws = q.ws + (size_t)grp * q.ws_stride;
-    MsCtl *ctl = reinterpret_cast<MsCtl *>(ws);
+    char *ctl_base = q.ws + (size_t)s_grp * WS_CONTROL_BYTES;
+    char *data = q.ws + q.groups[s_grp].data;
+    MsCtl *ctl = reinterpret_cast<MsCtl *>(ctl_base);
     unsigned epoch = 0;
-    while (true) {
-        if (GroupG::rank() == 0) ctl->item = atomicAdd(q.next, 1);
+    for (int own = q.groups[s_grp].first;; own = -1) {
+        if (GroupG::rank() == 0) ctl->item = own >= 0 ? own : atomicAdd(q.next, 1);
         if (!grid_barrier(&ctl->bar, &ctl->err, epoch, q.wait_ns, nullptr, nullptr, 0, (unsigned)GroupG::nblk())) return;
         if (threadIdx.x == 0) s_item = ld_volatile_i32(&ctl->item);
         __syncthreads();
@@ -1880,7 +1903,7 @@ __global__ void __launch_bounds__(MS_THREADS, MS_MIN_BLOCKS) ms_queue_kernel(MqA
             a.dist = m.dist;
             a.reach = m.reach;
             a.ld = m.ld;
-            ms_layout(ws, (size_t)m.n, W, a);
+            ms_layout(ctl_base, data, (size_t)m.n, W, a);
             a.alpha = q.alpha;
             a.beta = q.beta;
             a.gamma = q.gamma;
@@ -1989,7 +2012,7 @@ void launch_msbfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t *di
     a.dist = dist;
     a.reach = opt.reach;
     a.ld = ld;
-    ms_layout(ws, n, W, a);
+    ms_layout(ws, ws + WS_CONTROL_BYTES, n, W, a);
     a.alpha = opt.tuned ? opt.alpha : env_float("GU_MS_ALPHA", ms_size_alpha(opt.alpha, g.m));
     a.beta = opt.tuned ? opt.beta : env_float("GU_MS_BETA", opt.beta);
     a.gamma = env_float("GU_MS_GAMMA", opt.gamma);
@@ -2033,6 +2056,17 @@ static int queue_blocks_per_sm()
     return b;
 }
 
+// Estimated work of k sources of a request: passes over the vertices' words, over the
+// adjacency (a DAG's vertices are met again at several distances), the rows, and the
+// levels' fixed part.  The weights were varied by factors of two and more on four
+// request sets: the launch stayed within 2 % of the best but for cheaper DAGs or
+// dearer adjacencies (5-10 % longer).
+static double queue_weight(const MsQueueRequest &r, int32_t k)
+{
+    const double n = (double)r.g->n, m = (double)r.g->m;
+    return 1e7 + 3000.0 * n + (r.g->directed ? 500.0 : 50.0) * m + (r.dist ? 8.0 * n * k : 0.0);
+}
+
 // Words per vertex, groups and workspace of a work-queue launch over reqs.
 MsQueueLaunch msbfs_queue_plan(const std::vector<MsQueueRequest> &reqs, int sms, int max_blocks)
 {
@@ -2054,15 +2088,42 @@ MsQueueLaunch msbfs_queue_plan(const std::vector<MsQueueRequest> &reqs, int sms,
     const int bps = L.W == 1 ? queue_blocks_per_sm<1>() : L.W == 2 ? queue_blocks_per_sm<2>() : queue_blocks_per_sm<4>();
     int blocks = sms * bps;
     if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
-    // group size: about 16 K vertices per CTA of a group, larger while there are
-    // fewer items than groups, so that the grid is used
-    int gs = (int)std::min<size_t>((maxn + 16383) / 16384, (size_t)blocks);
-    gs = std::max(gs, std::max(1, blocks / L.items));
-    L.group_size = std::max(1, std::min(gs, blocks));
-    L.ngroups = blocks / L.group_size;
-    L.stride = ms_up256(ms_layout_bytes(maxn, L.W));
-    L.items_off = (size_t)L.ngroups * L.stride;
-    L.cnt_off = L.items_off + ms_up256(sizeof(MqItem) * (size_t)L.items);
+    size_t data = 0;  // workspace slices, after the control regions
+    if (2 * L.items <= blocks) {
+        std::vector<double> w;
+        std::vector<size_t> n;
+        double sum = 0;
+        for (const MsQueueRequest &r : reqs)
+            for (int32_t off = 0; off < r.k; off += per_item) {
+                w.push_back(queue_weight(r, std::min(per_item, r.k - off)));
+                n.push_back((size_t)r.g->n);
+                sum += w.back();
+            }
+        int base = 0;
+        for (size_t i = 0; i < w.size(); ++i) {
+            const int size = 1 + (int)((double)(blocks - L.items) * (w[i] / sum));
+            L.groups.push_back({base, size, (int)i, data});
+            base += size;
+            data += ms_up256(ms_data_bytes(n[i], L.W));
+        }
+        L.grid = std::min(base, blocks);
+        L.groups.back().size -= base - L.grid;  // (a rounding of the shares upwards, if any)
+        L.taken = L.items;
+    } else {
+        // equal groups: about 16 K vertices of the largest graph per CTA, larger while
+        // there are fewer items than groups
+        int gs = (int)std::min<size_t>((maxn + 16383) / 16384, (size_t)blocks);
+        gs = std::max(1, std::min(std::max(gs, blocks / L.items), blocks));
+        const size_t slice = ms_up256(ms_data_bytes(maxn, L.W));
+        for (int i = 0; i < blocks / gs; ++i, data += slice) L.groups.push_back({i * gs, gs, -1, data});
+        L.grid = (int)L.groups.size() * gs;
+        L.taken = 0;
+    }
+    const size_t ctl = L.groups.size() * WS_CONTROL_BYTES;
+    for (MsQueueLaunch::Group &g : L.groups) g.data += ctl;
+    L.items_off = ctl + data;
+    L.groups_off = L.items_off + ms_up256(sizeof(MqItem) * (size_t)L.items);
+    L.cnt_off = L.groups_off + ms_up256(sizeof(MqGroup) * L.groups.size());
     L.bytes = L.cnt_off + 256;
     return L;
 }
@@ -2106,17 +2167,23 @@ MsQueueLaunch launch_msbfs_queue(const std::vector<MsQueueRequest> &reqs, Worksp
         }
     }
     char *ws = (char *)wsp.get(L.bytes);
-    GU_CUDA_CHECK(cudaMemset2DAsync(ws, L.stride, 0, CTL_REGION, (size_t)L.ngroups, st));
-    GU_CUDA_CHECK(cudaMemsetAsync(ws + L.cnt_off, 0, sizeof(int), st));
-    GU_CUDA_CHECK(cudaMemcpyAsync(ws + L.items_off, items.data(), sizeof(MqItem) * items.size(), cudaMemcpyHostToDevice,
-                                  st));
+    GU_CUDA_CHECK(cudaMemset2DAsync(ws, WS_CONTROL_BYTES, 0, CTL_REGION, L.groups.size(), st));
+    // items, groups and the counter are neighbours: one copy
+    std::vector<char> head(L.cnt_off + sizeof(int) - L.items_off);
+    std::memcpy(head.data(), items.data(), sizeof(MqItem) * items.size());
+    for (size_t i = 0; i < L.groups.size(); ++i) {
+        const MqGroup g = {L.groups[i].base, L.groups[i].size, L.groups[i].first, 0, (u64)L.groups[i].data};
+        std::memcpy(head.data() + (L.groups_off - L.items_off) + i * sizeof(MqGroup), &g, sizeof(MqGroup));
+    }
+    std::memcpy(head.data() + (L.cnt_off - L.items_off), &L.taken, sizeof(int));
+    GU_CUDA_CHECK(cudaMemcpyAsync(ws + L.items_off, head.data(), head.size(), cudaMemcpyHostToDevice, st));
     MqArgs q;
     q.items = reinterpret_cast<const MqItem *>(ws + L.items_off);
     q.nitems = (int)items.size();
     q.next = reinterpret_cast<int *>(ws + L.cnt_off);
     q.ws = ws;
-    q.ws_stride = L.stride;
-    q.group_size = L.group_size;
+    q.groups = reinterpret_cast<const MqGroup *>(ws + L.groups_off);
+    q.ngroups = (int)L.groups.size();
     // a group's barrier is cheap next to the whole grid's: no size rule here (24 requests
     // of the serving mix: 1429 us, with ms_size_alpha and ms_size_rare 1464 us)
     q.alpha = env_float("GU_MS_ALPHA", MS_ALPHA);
@@ -2127,7 +2194,7 @@ MsQueueLaunch launch_msbfs_queue(const std::vector<MsQueueRequest> &reqs, Worksp
     void *params[] = {&q};
     const void *fn = W == 1 ? (const void *)ms_queue_kernel<1> : W == 2 ? (const void *)ms_queue_kernel<2>
                                                                        : (const void *)ms_queue_kernel<4>;
-    GU_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3(L.ngroups * L.group_size), dim3(MS_THREADS), params, 0, st));
+    GU_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3(L.grid), dim3(MS_THREADS), params, 0, st));
     return L;
 }
 
@@ -2135,10 +2202,10 @@ MsQueueLaunch launch_msbfs_queue(const std::vector<MsQueueRequest> &reqs, Worksp
 // its stream is synchronised).
 int msbfs_queue_error(const Workspace &ws, const MsQueueLaunch &L)
 {
-    if (L.ngroups == 0) return 0;
-    std::vector<int> e((size_t)L.ngroups, 0);
-    GU_CUDA_CHECK(cudaMemcpy2D(e.data(), sizeof(int), static_cast<const char *>(ws.ptr) + offsetof(MsCtl, err), L.stride,
-                               sizeof(int), (size_t)L.ngroups, cudaMemcpyDeviceToHost));
+    if (L.groups.empty()) return 0;
+    std::vector<int> e(L.groups.size(), 0);
+    GU_CUDA_CHECK(cudaMemcpy2D(e.data(), sizeof(int), static_cast<const char *>(ws.ptr) + offsetof(MsCtl, err),
+                               WS_CONTROL_BYTES, sizeof(int), e.size(), cudaMemcpyDeviceToHost));
     for (int x : e)
         if (x) return x;
     return 0;
