@@ -181,6 +181,7 @@ struct DeviceGraph {
     void *ctl_host = nullptr;  // pinned copy of the batched engine's control block, written after each launch
     int32_t *ell = nullptr;  // low-degree graphs: neighbours padded to ell_width per vertex (-1), built on first use
     int ell_width = 0;
+    bool local_wide = false;  // per-source engine: a search overflowed its smaller ring
     // bottom-up degree classes by in-degree, each ascending: light (1 ..
     // BU_LIGHT_DEGREE), mid (.. BU_MID_DEGREE), wide (.. BU_HEAVY_DEGREE),
     // heavy (above)
