@@ -32,6 +32,7 @@
 // order.  The result depends on the grid size, which the graph and k fix, and not on
 // scheduling.
 #include "device_utils.cuh"
+#include "fp64_int.cuh"
 #include "gu_internal.h"
 
 #include <algorithm>
@@ -72,25 +73,6 @@ __host__ __device__ inline size_t sc_smem_bytes(int n)
     return v * (sizeof(u64) + 4 * sizeof(uint16_t));
 }
 
-// A sum of positive doubles: acc in units of 2^(e - 1023 - 52 - G), e the largest
-// (biased) exponent added, each term rounded to nearest; at most 2^(11 - G) - 1 terms.
-template <int G>
-struct IntSum {
-    u64 acc = 0;
-    int e = 0;
-    __device__ __forceinline__ void add(double x)
-    {
-        const u64 b = (u64)__double_as_longlong(x);
-        const int ex = (int)(b >> 52);
-        u64 m = ((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << G;
-        const int up = max(ex - e, 0), down = max(e - ex, 0);
-        acc = up < 64 ? acc >> up : 0ull;  // (the dropped bits: less than a unit, once per new largest term)
-        e = max(e, ex);
-        m = down < 60 ? (m + ((1ull << down) >> 1)) >> down : 0ull;
-        acc += m;
-    }
-    __device__ __forceinline__ double value() const { return acc ? scalbn((double)acc, e - 1023 - 52 - G) : 0.0; }
-};
 constexpr int SC_GUARD_LANE = 4;  // up to 127 terms: a short list
 constexpr int SC_GUARD_WARP = 3;  // up to 255: a lane's share of a list of 32 x 255
 constexpr int SC_MAX_DEGREE = 32 * 255;
@@ -232,14 +214,14 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
             __syncthreads();
             const double *beta = reinterpret_cast<const double *>(val);
             auto finish = [&](int w, double S) {
-                const double sg = (double)val[w], d = sg * S;
-                reinterpret_cast<double *>(val)[w] = (1.0 + d) / sg;
+                const double sg = u64_to_double(val[w]), d = sg * S;
+                reinterpret_cast<double *>(val)[w] = quotient(1.0 + d, sg);
                 __stcg(part + w, __ldcg(part + w) + d);
                 if (drow) drow[__ldg(a.oldid + w)] = d;
             };
             for (int i = lstart[L] + threadIdx.x; L > 0 && i < lstart[L + 1]; i += T) {  // no successors
                 const int w = ord[i];
-                reinterpret_cast<double *>(val)[w] = 1.0 / (double)val[w];
+                reinterpret_cast<double *>(val)[w] = quotient(1.0, u64_to_double(val[w]));
             }
             __syncthreads();
             for (int l = L - 1; l >= 1; --l) {
@@ -402,9 +384,9 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
 }
 
 // Whether gu_bc / gu_sigma take this engine.  Call times in us, this engine / the
-// batched one: ER 198 k = 198 53 / 236, ER 4000 k = 256 169 / 299, R-MAT 10 k = 256
-// 90 / 756, R-MAT 12 k = 1024 655 / 1360 (1024 sources per pass; 3980 at the default
-// 256), R-MAT 13 k = 1024 1487 / 1676 (4335).  Above 8192 vertices the state does not
+// batched one: ER 198 k = 198 60 / 225, ER 4000 k = 256 156 / 299, R-MAT 10 k = 256
+// 107 / 756, R-MAT 12 k = 1024 664 / 1360 (1024 sources per pass; 3980 at the default
+// 256), R-MAT 13 k = 1024 1474 / 1676 (4335).  Above 8192 vertices the state does not
 // fit an SM.  A batch narrower than the request asks for passes, which only the batched
 // engine has.
 bool smem_bc_takes(const DeviceGraph &g, int32_t k, int32_t batch)
