@@ -376,7 +376,11 @@ __device__ __forceinline__ void finish_delta(const BcArgs &a, size_t o, double S
 // instruction adds 32 of them.  Each source still receives its successors'
 // terms one at a time in CSR order (a successor's list holds a source at most
 // once, and successive lists are separated by __syncwarp), so the sums are the
-// sequential CSR-order sums.
+// sequential CSR-order sums.  The lists of four successors are made together, a lane per
+// 32-bit word of a mask (a successor at a time, by ballots' ranks, cost 72 instructions
+// each: R-MAT18, 1024 sources, levels 1 / 2 / 3 took 2.34 / 6.14 / 3.85 ms, now 1.58 /
+// 5.48 / 3.13; six or eight rounds of loads in flight instead of four are slower, 5.63
+// and 6.07 ms on level 2).
 template <int NQ>
 struct SumStage {
     double acc[64 * NQ];
@@ -406,6 +410,7 @@ __device__ __forceinline__ int compact_bits(const u64 (&m)[NQ], unsigned char *l
 template <int NQ>
 __device__ void bc_backward_item(const BcArgs &a, EdgeStage<NQ> &st, SumStage<NQ> &ss, int l, int L, int q0, int c)
 {
+    constexpr int WPS = 2 * NQ;  // 32-bit words per successor
     const int lane = lane_id();
     const int W = a.W, B = 64 * W;
     const size_t nW = (size_t)a.n * W;
@@ -437,36 +442,48 @@ __device__ void bc_backward_item(const BcArgs &a, EdgeStage<NQ> &st, SumStage<NQ
             while (bal) {  // up to four successors at a time, in CSR order
                 int src[4];
                 next_lanes<4>(bal, src);
-                int cnt[4], cum[4], rounds = 0;
+                // lane t lists the set bits of 32-bit word h of successor u
+                const int u = lane / WPS, h = lane % WPS;
+                const int su = u == 0 ? src[0] : u == 1 ? src[1] : u == 2 ? src[2] : u == 3 ? src[3] : -1;
+                unsigned x = su < 0 ? 0u : reinterpret_cast<const unsigned *>(&st.m[h >> 1][su])[h & 1];
+                const int own = __popc(x);
+                int upto = own;  // bits in the successor's words up to this one
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    cnt[u] = 0;
-                    if (src[u] >= 0) {
-                        u64 mm[NQ];
-#pragma unroll
-                        for (int t = 0; t < NQ; ++t) mm[t] = st.m[t][src[u]];
-                        cnt[u] = compact_bits<NQ>(mm, ss.pos[u]);
-                    }
-                    rounds += (cnt[u] + 31) >> 5;
-                    cum[u] = rounds;
+                for (int o = 1; o < WPS; o <<= 1) {
+                    const int y = __shfl_up_sync(FULL_MASK, upto, o, WPS);
+                    if (h >= o) upto += y;
                 }
+                unsigned char *out = ss.pos[0] + 64 * NQ * u + upto - own;
+                while (x) {
+                    *out++ = (unsigned char)(32 * h + __ffs(x) - 1);
+                    x &= x - 1;
+                }
+                // rounds of 32 sources of one successor; lane r describes round r
+                int rounds = 0, at = 0, left = 0, v = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int cnt = __shfl_sync(FULL_MASK, upto, WPS * k + WPS - 1), r = lane - rounds;
+                    if (r >= 0 && src[k] >= 0) {
+                        at = 64 * NQ * k + 32 * r;
+                        left = cnt - 32 * r;
+                        v = st.v[src[k]];
+                    }
+                    rounds += (cnt + 31) >> 5;
+                }
+                const int desc = lane < rounds ? at | min(left, 32) << 16 : 0;
                 __syncwarp();
                 for (int r0 = 0; r0 < rounds; r0 += 4) {
                     double b[4];
                     int s[4];
 #pragma unroll
                     for (int z = 0; z < 4; ++z) {  // four loads in flight per lane
-                        const int rr = r0 + z;
-                        const int u = (rr >= cum[0]) + (rr >= cum[1]) + (rr >= cum[2]);
-                        const int first = u == 0 ? 0 : u == 1 ? cum[0] : u == 2 ? cum[1] : cum[2];
-                        const int n_u = u == 0 ? cnt[0] : u == 1 ? cnt[1] : u == 2 ? cnt[2] : cnt[3];
-                        const int s_u = u == 0 ? src[0] : u == 1 ? src[1] : u == 2 ? src[2] : src[3];
-                        const int i = 32 * (rr - first) + lane;
+                        const int rr = (r0 + z) & 31;  // r0 + z < 32 where there is such a round
+                        const int dz = __shfl_sync(FULL_MASK, desc, rr), vz = __shfl_sync(FULL_MASK, v, rr);
                         s[z] = -1;
                         b[z] = 0.0;
-                        if (rr < rounds && i < n_u) {
-                            s[z] = ss.pos[u][i];
-                            b[z] = __ldcg(bet + (size_t)st.v[s_u] * B + s[z]);
+                        if (lane < dz >> 16) {
+                            s[z] = ss.pos[0][(dz & 0xFFFF) + lane];
+                            b[z] = __ldcg(bet + (size_t)vz * B + s[z]);
                         }
                     }
 #pragma unroll
