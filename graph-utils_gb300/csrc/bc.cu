@@ -376,15 +376,17 @@ __device__ __forceinline__ void finish_delta(const BcArgs &a, size_t o, double S
 // instruction adds 32 of them.  Each source still receives its successors'
 // terms one at a time in CSR order (a successor's list holds a source at most
 // once, and successive lists are separated by __syncwarp), so the sums are the
-// sequential CSR-order sums.  The lists of four successors are made together, a lane per
-// 32-bit word of a mask (a successor at a time, by ballots' ranks, cost 72 instructions
-// each: R-MAT18, 1024 sources, levels 1 / 2 / 3 took 2.34 / 6.14 / 3.85 ms, now 1.58 /
+// sequential CSR-order sums.  The lists of SUCC successors are made together, a lane per
+// 32-bit word of a mask (a successor at a time, by ranks, cost 72 instructions each: R-MAT18, 1024 sources, levels 1 / 2 / 3 took 2.34 / 6.14 / 3.85 ms, now 1.58 /
 // 5.48 / 3.13; six or eight rounds of loads in flight instead of four are slower, 5.63
 // and 6.07 ms on level 2).
 template <int NQ>
 struct SumStage {
     double acc[64 * NQ];
-    unsigned char pos[4][64 * NQ];  // dense source lists of up to four successors
+    static constexpr int SUCC = 16 / NQ;  // as many successors as have 32 words of 32 bits
+    unsigned char pos[SUCC][64 * NQ];     // dense source lists of their bits
+    int2 round[32];                       // first list position | entries << 16, successor
+    unsigned char edge[32];               // the slice's edges with work
 };
 
 // Writes the positions (0 .. 64*NQ-1) of the set bits of m into list in
@@ -410,7 +412,7 @@ __device__ __forceinline__ int compact_bits(const u64 (&m)[NQ], unsigned char *l
 template <int NQ>
 __device__ void bc_backward_item(const BcArgs &a, EdgeStage<NQ> &st, SumStage<NQ> &ss, int l, int L, int q0, int c)
 {
-    constexpr int WPS = 2 * NQ;  // 32-bit words per successor
+    constexpr int WPS = 2 * NQ, SUCC = SumStage<NQ>::SUCC;  // 32-bit words per successor
     const int lane = lane_id();
     const int W = a.W, B = 64 * W;
     const size_t nW = (size_t)a.n * W;
@@ -437,15 +439,16 @@ __device__ void bc_backward_item(const BcArgs &a, EdgeStage<NQ> &st, SumStage<NQ
                 st.v[lane] = v;
                 any = any_bits(m);
             }
-            unsigned bal = __ballot_sync(FULL_MASK, any);
+            const unsigned bal = __ballot_sync(FULL_MASK, any);
+            const int total = __popc(bal);
+            if (any) ss.edge[__popc(bal & ((1u << lane) - 1u))] = (unsigned char)lane;
             __syncwarp();
-            while (bal) {  // up to four successors at a time, in CSR order
-                int src[4];
-                next_lanes<4>(bal, src);
+            for (int i0 = 0; i0 < total; i0 += SUCC) {  // SUCC successors at a time, in CSR order
                 // lane t lists the set bits of 32-bit word h of successor u
                 const int u = lane / WPS, h = lane % WPS;
-                const int su = u == 0 ? src[0] : u == 1 ? src[1] : u == 2 ? src[2] : u == 3 ? src[3] : -1;
-                unsigned x = su < 0 ? 0u : reinterpret_cast<const unsigned *>(&st.m[h >> 1][su])[h & 1];
+                const bool on = i0 + u < total;
+                const int su = on ? ss.edge[i0 + u] : 0;
+                unsigned x = on ? reinterpret_cast<const unsigned *>(&st.m[h >> 1][su])[h & 1] : 0u;
                 const int own = __popc(x);
                 int upto = own;  // bits in the successor's words up to this one
 #pragma unroll
@@ -453,25 +456,24 @@ __device__ void bc_backward_item(const BcArgs &a, EdgeStage<NQ> &st, SumStage<NQ
                     const int y = __shfl_up_sync(FULL_MASK, upto, o, WPS);
                     if (h >= o) upto += y;
                 }
-                unsigned char *out = ss.pos[0] + 64 * NQ * u + upto - own;
+                unsigned char *out = ss.pos[u] + upto - own;
                 while (x) {
                     *out++ = (unsigned char)(32 * h + __ffs(x) - 1);
                     x &= x - 1;
                 }
-                // rounds of 32 sources of one successor; lane r describes round r
-                int rounds = 0, at = 0, left = 0, v = 0;
+                // rounds of 32 sources of one successor: its lane h describes its round h
+                const int cnt = __shfl_sync(FULL_MASK, upto, WPS - 1, WPS), mine = (cnt + 31) >> 5;
+                int last = mine;  // rounds up to this successor's last
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int cnt = __shfl_sync(FULL_MASK, upto, WPS * k + WPS - 1), r = lane - rounds;
-                    if (r >= 0 && src[k] >= 0) {
-                        at = 64 * NQ * k + 32 * r;
-                        left = cnt - 32 * r;
-                        v = st.v[src[k]];
-                    }
-                    rounds += (cnt + 31) >> 5;
+                for (int o = WPS; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(FULL_MASK, last, o);
+                    if (lane >= o) last += y;
                 }
-                const int desc = lane < rounds ? at | min(left, 32) << 16 : 0;
+                if (h < mine)
+                    ss.round[last - mine + h] = make_int2((64 * NQ * u + 32 * h) | min(cnt - 32 * h, 32) << 16, st.v[su]);
+                const int rounds = __shfl_sync(FULL_MASK, last, 31);
                 __syncwarp();
+                const int desc = lane < rounds ? ss.round[lane].x : 0, v = lane < rounds ? ss.round[lane].y : 0;
                 for (int r0 = 0; r0 < rounds; r0 += 4) {
                     double b[4];
                     int s[4];
