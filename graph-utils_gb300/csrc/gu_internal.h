@@ -28,6 +28,8 @@ constexpr int BU_MID_DEGREE = 32;
 constexpr int BU_HEAVY_DEGREE = 128;
 // AUTO takes the per-source engine with shared-memory queues up to this out-degree.
 constexpr int LOCAL_MAX_DEGREE = 16;
+// ... ahead of the shared-memory engine up to this one.
+constexpr int LOCAL_MESH_DEGREE = 4;
 // Every workspace starts with this many bytes of launch control block and
 // profiling timeline; kernel scratch follows.
 constexpr size_t WS_CONTROL_BYTES = 65536;

@@ -58,6 +58,7 @@ struct LocalArgs {
     int *max_level;             // atomicMax of the deepest level reached (null: none)
     int *overflow;              // set when a frontier exceeds the queue
     int ring;                   // entries of local_bfs_kernel's ring
+    bool alone;                 // one CTA per SM: local_bfs_kernel keeps adjacency pieces in L1
 };
 
 __global__ void build_ell_kernel(const int32_t *__restrict__ R, const int32_t *__restrict__ C, int32_t n, int width,
@@ -86,9 +87,11 @@ constexpr unsigned RECENT_EMPTY = 0xFFFFu;  // a vertex with this tag always goe
 static_assert(RECENT_BITS + 16 == 30, "slot and tag cover the 30-bit hash");
 __device__ __forceinline__ uint32_t recent_hash(int32_t v) { return ((uint32_t)v * 0x2C1B3C6Du) & 0x3FFFFFFFu; }
 
-// A piece of an adjacency row, kept out of L1: every lane reads another line, and lines
-// in flight that fill the L1 hold up the claims (2048 x 2048 grid, 256 sources: 35.0 ->
-// 34.2 ms; with 8 KiB more shared memory, so less L1, 37.1).
+// A piece of an adjacency row, kept out of L1: every lane reads another line, and with
+// two CTAs on an SM lines in flight that fill the L1 hold up the claims (2048 x 2048
+// grid, 256 sources: 35.0 -> 34.2 ms; with 8 KiB more shared memory, so less L1, 37.1).
+// A CTA alone on its SM keeps them: a line's other vertices come up on the next levels
+// (1024 x 1024, 64 sources, counts 6.4 ms past L1, 6.2 through it).
 __device__ __forceinline__ int4 ld_row(const int4 *p)
 {
     int4 q;
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(LOCAL_THREADS, 2) local_bfs_kernel(LocalArgs a
                 bool go = on;
 #pragma unroll
                 for (int c = 0; c < WIDTH / 4; ++c) {
-                    const int4 q4 = go ? ld_row(row + c) : make_int4(-1, -1, -1, -1);
+                    const int4 q4 = go ? (a.alone ? __ldg(row + c) : ld_row(row + c)) : make_int4(-1, -1, -1, -1);
                     const int32_t w[4] = {q4.x, q4.y, q4.z, q4.w};
                     go = w[0] >= 0;  // padding: the list ended
                     if (!__any_sync(FULL_MASK, go)) break;
@@ -228,11 +231,20 @@ constexpr int MESH_ROWS = 1536;                 // rows per shared queue (two: 4
 constexpr int MESH_QCAP = 4 * MESH_ROWS;        // ids in the same space; wider levels go back to the caller
 constexpr int MESH_NARROW = MESH_ROWS / 4;      // every neighbour reserved: no overflow of the rows
 constexpr int MESH_RECENT_BITS = 12;
-// Larger meshes are wide on most levels and take local_bfs_kernel.  1024 x 1024 grid: rows
-// of 1 / 64 / 256 sources 4.48 / 5.81 / 8.29 ms here, 6.01 / 7.64 / 9.24 there; counts
-// 6.23 / 7.04 / 9.61 here, 6.10 / 6.33 / 7.33 there.  2048 x 2048, 256 sources: rows 41.6
-// here, 34.9 there.  724 x 724, 256 sources, counts: 4.46 here.
-constexpr int MESH_MAX_N_ROWS = 1 << 20, MESH_MAX_N_COUNT = 1 << 19;
+// Meshes on which two CTAs share an SM and most levels are wide take local_bfs_kernel.
+// Rows, here / there: 1024 x 1024 grid, 1 / 64 / 256 sources 4.8 / 5.6 / 8.4 ms and 6.0 /
+// 7.6 / 9.2; 876 x 1763, 64 / 256 sources 7.5 / 11.6 and 10.2 / 13.3; 2048 x 2048, 64 /
+// 150 / 256 sources 20.3 / 22.0 / 40.6 and 23.2 / 25.7 / 35.7.  Counts, where a claim is
+// in a small bitmap and the chain is shorter: 600 x 1000, 1 / 64 / 256 sources 3.6 / 3.7 /
+// 5.2 and 3.4 / 4.2 / 5.0; 863 x 642 2.9 / 3.4 / 4.7 and 3.2 / 4.2 / 4.7; 1024 x 1024 6.7
+// / 6.8 / 9.7 and 5.7 / 6.2 / 7.5.  (A long narrow mesh of this size would do better here:
+// 300 x 6000, 64 sources, counts 12.2 and 17.6.)
+constexpr int MESH_MAX_N_SHARED = 1 << 21, MESH_MAX_N_COUNT = 5 << 17;
+static bool mesh_form(const DeviceGraph &g, int32_t k, bool rows)
+{
+    if (g.ell_width != LOCAL_MESH_DEGREE) return false;
+    return rows ? k <= g.sm_count || g.n <= MESH_MAX_N_SHARED : g.n <= MESH_MAX_N_COUNT;
+}
 constexpr size_t MESH_SMEM = 2 * MESH_ROWS * sizeof(int4) + sizeof(int32_t) * (1 << MESH_RECENT_BITS);
 
 __device__ __forceinline__ void copy16_async(void *dst, const void *src)
@@ -406,7 +418,7 @@ bool launch_local_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
         GU_CUDA_CHECK(cudaGetLastError());
     }
     const bool rows = dist != nullptr;
-    const int wi = g.ell_width == 8 ? 1 : g.ell_width == 16 ? 2 : g.n <= (rows ? MESH_MAX_N_ROWS : MESH_MAX_N_COUNT) ? 3 : 0;
+    const int wi = g.ell_width == 8 ? 1 : g.ell_width == 16 ? 2 : mesh_form(g, k, rows) ? 3 : 0;
     const bool mesh = wi == 3;
     void (*const kerns[2][4])(LocalArgs) = {{local_bfs_kernel<false, 4>, local_bfs_kernel<false, 8>,
                                              local_bfs_kernel<false, 16>, mesh_bfs_kernel<false>},
@@ -444,6 +456,7 @@ bool launch_local_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
     a.max_level = reinterpret_cast<int *>(ws);
     a.overflow = reinterpret_cast<int *>(ws) + 1;
     a.ring = ring;
+    a.alone = grid <= g.sm_count;
     g.timeline = 0;
     g.mark_start(stream);
     kern<<<grid, LOCAL_THREADS, smem, stream>>>(a);

@@ -660,6 +660,10 @@ static SbConfig sb_config(const DeviceGraph &g, int S, int threads)
 //     counts, k = 100, one CTA a source: 451 / 305), and beyond 131072 vertices, where
 //     a source needs eight CTAs, up to 8 sources (R-MAT 18 k = 8 115 / 153, k = 16 179 /
 //     167).
+// Out-degrees up to four go to the mesh form of the per-source engine (rows, this engine
+// / that one: 48 x 48 grid k = 1 183 / 128 us, 100 x 100 k = 150 488 / 313, 128 x 128
+// k = 256 718 / 410); with out-degrees of 5 to 16 this one is ahead (random graph of 10000
+// vertices, k = 64, 75 / 139).
 // Cluster size: as many CTAs per source as all k keep resident at once, while a CTA
 // has at least 4096 vertices (R-MAT 17 k = 1: S = 4 83 us, 8 65, 16 58; R-MAT 14
 // k = 1: S = 1 47, 4 43, 16 43).
@@ -669,7 +673,7 @@ static SbConfig sb_choose(const DeviceGraph &g, int32_t k)
     if (e && e[0] == '0') return SbConfig();  // AUTO kept on the batched engine
     const double km = (double)k * (double)g.m;
     const bool low = g.max_degree <= LOCAL_MAX_DEGREE, many = k > g.sm_count;
-    if (k < 1 || g.n < 1 || g.m > SB_MAX_M) return SbConfig();
+    if (k < 1 || g.n < 1 || g.m > SB_MAX_M || g.max_degree <= LOCAL_MESH_DEGREE) return SbConfig();
     if (g.n <= 16384) {
         if (low && many && g.n <= 8192) return SbConfig();
     } else if (low) {
