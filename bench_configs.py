@@ -152,7 +152,7 @@ def source_hash(files):
     return h.hexdigest()[:16]
 
 
-BC_SOURCES = ("bc.cu", "device_utils.cuh", "gu_internal.h")
+BC_SOURCES = ("bc.cu", "device_utils.cuh", "fp64_int.cuh", "gu_internal.h")
 
 
 def bc_subline(torch):
@@ -341,7 +341,7 @@ def wl_c3(args):
            "roofline": {"bound": "hbm", "alg_bytes": alg, "achieved_gbs": alg / best / 1e6,
                         "peak_gbs": _hbm_peak(), "effective_frac": alg / best / 1e6 / _hbm_peak(),
                         "model": "per-source 28n + 32 V_s + 40 E_s (effective: a pass shares reads)",
-                        "physical": "ncu of one 256-source pass: 9.87 GB DRAM in 6.32 ms, 1.56 TB/s, 0.23 of "
+                        "physical": "ncu of the 1024-per-pass launch: 322 GB DRAM in 140 ms, 2.29 TB/s, 0.34 of "
                                     "the measured HBM peak (profiles/bc_grid_kernel_rmat18.md)"},
            "cpu_bc_f64": {"per_source_ms_1thread": c1 * 1e3 / len(sub1),
                           f"per_source_ms_{cores}threads": cN * 1e3 / len(subN),
