@@ -26,6 +26,7 @@
 // chain.
 #include "device_utils.cuh"
 #include "gu_internal.h"
+#include "recent.h"
 
 #include <algorithm>
 #include <climits>
@@ -73,19 +74,16 @@ __global__ void build_ell_kernel(const int32_t *__restrict__ R, const int32_t *_
 }
 
 // Vertices claimed lately by the CTA's search: a direct-mapped table of 16-bit tags in
-// shared memory.  The hash is a bijection of 30-bit ids, slot its upper and tag its
-// lower bits, so a tag that matches is this vertex and no other; a tag that was
-// overwritten only sends the vertex to the global claim again.  A mesh vertex's
+// shared memory.  The hash is a bijection of the ids below 2^30, slot its upper and tag
+// its lower bits, so a tag that matches is this vertex and no other; a tag that was
+// overwritten only sends the vertex to the global claim again, and an id from 2^30 up
+// always goes there.  A mesh vertex's
 // neighbours lie on the levels before and after its own, so nearly all that are
 // claimed already were claimed within two levels and are found here: a shared-memory
 // read whose lanes meet a few bank conflicts, where a read of the distance row or the
 // bitmap is a line of its own for every lane (2048 x 2048 grid, 256 sources: rows 40.6 ->
 // 37.1 ms, counts 34.9 -> 30.2; 2^13 slots 37.6, 2^12 42).
-constexpr int RECENT_BITS = 14;
-constexpr int RECENT_SLOTS = 1 << RECENT_BITS;
-constexpr unsigned RECENT_EMPTY = 0xFFFFu;  // a vertex with this tag always goes to the global claim
-static_assert(RECENT_BITS + 16 == 30, "slot and tag cover the 30-bit hash");
-__device__ __forceinline__ uint32_t recent_hash(int32_t v) { return ((uint32_t)v * 0x2C1B3C6Du) & 0x3FFFFFFFu; }
+// (The constants and the hash: recent.h.)
 
 // A piece of an adjacency row, kept out of L1: every lane reads another line, and with
 // two CTAs on an SM lines in flight that fill the L1 hold up the claims (2048 x 2048
