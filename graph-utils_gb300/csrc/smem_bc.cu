@@ -353,8 +353,9 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
     uint16_t *newid = reinterpret_cast<uint16_t *>(host.data() + r_bytes);
     uint16_t *oldid = reinterpret_cast<uint16_t *>(host.data() + r_bytes + id_bytes);
     const std::vector<int32_t> &R = g.host_R;
-    // counting sort by descending out-degree (longer lists than n together first)
-    const int32_t top = (int32_t)n;
+    // counting sort by descending out-degree (longer lists than top together first); with
+    // parallel edges a list can be longer than n, and the long ones still come first
+    const int32_t top = std::max((int32_t)n, SC_LONG);
     std::vector<int32_t> at((size_t)top + 2, 0);
     auto key = [&](size_t v) { return top - std::min(R[v + 1] - R[v], top); };
     for (size_t v = 0; v < n; ++v) ++at[(size_t)key(v) + 1];

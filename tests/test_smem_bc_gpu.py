@@ -107,3 +107,18 @@ def test_bad_sources_and_batches():
         g.bc(s, bc, batch=batch)
         assert (g.level_profile() == []) == (batch != 64)
         np.testing.assert_allclose(bc.cpu().numpy(), ref, rtol=RTOL, atol=0)
+
+
+def test_parallel_edges_on_few_vertices():
+    """Lists longer than the graph has vertices (parallel edges are kept): those of 64
+    entries and more come first in a level whatever n is, so that no lane sums a list
+    longer than its integer sum has room for."""
+    n, rng = 40, np.random.default_rng(9)
+    # layers 0 | 1 .. 20 | 21 .. 39: lists of 40 .. 60 and of 300 entries in one level, the
+    # longer ones behind
+    reps = np.where(np.arange(20) % 3 == 2, 300, rng.integers(40, 60, 20))
+    R = np.zeros(n + 1, np.int32)
+    lists = [np.arange(1, 21)] + [np.sort(rng.integers(21, 40, r)) for r in reps] + [np.zeros(0, np.int64)] * 19
+    R[1:] = np.cumsum([len(x) for x in lists])
+    hg = gu.HostGraph(R, np.concatenate(lists).astype(np.int32), n, directed=True)
+    check(hg, np.resize(np.arange(n, dtype=np.int32), 640), directed=True)
