@@ -76,6 +76,9 @@ __host__ __device__ inline size_t sc_smem_bytes(int n)
 constexpr int SC_GUARD_LANE = 4;  // up to 127 terms: a short list
 constexpr int SC_GUARD_WARP = 3;  // up to 255: a lane's share of a list of 32 x 255
 constexpr int SC_MAX_DEGREE = 32 * 255;
+// IntSum::e from which a term was infinite or NaN (a count that wrapped to zero: beta is
+// 1 / 0): the sum is then formed by FP64 additions, which have a result for those.
+constexpr int SC_NOT_FINITE = 2047;
 
 __device__ __forceinline__ void shared_add_u64(u64 *p, u64 x)
 {
@@ -242,6 +245,21 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
                             if (lev[v] == next) s.add(beta[v]);
                         }
                         const int em = __reduce_max_sync(FULL_MASK, s.e), d = em - s.e;
+                        if (em >= SC_NOT_FINITE) {  // warp-uniform
+                            double p = 0.0;
+                            for (int32_t e = __ldg(a.R + w) + lane; e < e1; e += 32) {
+                                const unsigned v = __ldg(a.C + e);
+                                if (lev[v] == next) p += beta[v];
+                            }
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(FULL_MASK, p, o);
+                            if (lane == j) {
+                                khi = (u64)__double_as_longlong(p);
+                                ke = em;
+                                kw = w;
+                            }
+                            continue;
+                        }
                         // acc 2^24, shifted to the largest exponent: 96 bits, 32 of them add up
                         u64 hi = d < 56 ? s.acc >> (d + 8) : 0ull;
                         unsigned lo = d <= 24 ? (unsigned)(s.acc << (24 - d)) : d < 88 ? (unsigned)(s.acc >> (d - 24)) : 0u;
@@ -259,7 +277,9 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
                             kw = w;
                         }
                     }
-                    if (kw >= 0) {
+                    if (kw >= 0 && ke >= SC_NOT_FINITE) {
+                        finish(kw, __longlong_as_double((long long)khi));
+                    } else if (kw >= 0) {
                         const double x = (double)khi * 4294967296.0 + (double)klo;
                         finish(kw, x == 0.0 ? 0.0 : scalbn(x, ke - 1023 - 52 - SC_GUARD_WARP - 24));
                     }
@@ -278,7 +298,15 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
                             if (e + t >= e0 && e + t < e1 && lev[v] == next) s.add(beta[v]);
                         }
                     }
-                    finish(w, s.value());
+                    double S = s.value();
+                    if (s.e >= SC_NOT_FINITE) {
+                        S = 0.0;
+                        for (int32_t e = e0; e < e1; ++e) {
+                            const unsigned v = __ldg(a.C + e);
+                            if (lev[v] == next) S += beta[v];
+                        }
+                    }
+                    finish(w, S);
                 }
                 __syncthreads();
             }
@@ -324,7 +352,7 @@ __global__ void __launch_bounds__(256) smem_bc_reduce_kernel(const double *__res
             add_exactly(t, c, s[i][x]);
             c += sc[i][x];
         }
-        bc[__ldg(oldid + v)] = t + c;
+        bc[__ldg(oldid + v)] = isfinite(t) ? t + c : t;  // (the roundings' errors of an infinite sum are NaN)
     }
 }
 

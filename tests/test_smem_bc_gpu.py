@@ -122,3 +122,34 @@ def test_parallel_edges_on_few_vertices():
     R[1:] = np.cumsum([len(x) for x in lists])
     hg = gu.HostGraph(R, np.concatenate(lists).astype(np.int32), n, directed=True)
     check(hg, np.resize(np.arange(n, dtype=np.int32), 640), directed=True)
+
+
+@pytest.mark.parametrize("widths,what", [([1] + [2] * 65 + [200, 50, 10, 80, 3], np.isnan),
+                                         ([1] + [2] * 65, np.isinf), ([1] + [2] * 63 + [100, 2], np.isinf)])
+def test_counts_that_wrap_to_zero(widths, what):
+    """2^64 paths wrap to a count of zero: 1 / 0 is infinite (where the search ends there)
+    and 0 x inf NaN from there up.  Each dependency and betweenness must be the same
+    number, infinity or NaN as the batched engine's; in lists that a warp sums (80 and 200
+    entries) and that a lane does."""
+    start = np.concatenate([[0], np.cumsum(widths)])
+    u, v = [], []
+    for i in range(len(widths) - 1):
+        a, b = np.meshgrid(np.arange(start[i], start[i + 1]), np.arange(start[i + 1], start[i + 2]))
+        u.append(a.ravel())
+        v.append(b.ravel())
+    for symmetric in (False, True):
+        hg = gu.HostGraph.from_edges(int(start[-1]), np.concatenate(u), np.concatenate(v), symmetric=symmetric)
+        g = gu.Graph(hg)
+        srcs = np.resize([v for v in (0, 1, 2, 3, 5, 131, 140, 400, hg.n - 1) if v < hg.n], 70).astype(np.int32)
+        s = torch.as_tensor(srcs, device="cuda")
+        out = []
+        for batch in (0, 64):
+            bc = torch.empty(hg.n, dtype=torch.float64, device="cuda")
+            delta = torch.full((len(srcs), hg.n), -7.0, dtype=torch.float64, device="cuda")
+            g.bc(s, bc, delta_dev=delta, batch=batch)
+            assert (g.level_profile() == []) == (batch == 0)
+            out.append((bc.cpu().numpy(), delta.cpu().numpy()))
+        assert symmetric or what(out[1][1]).any()
+        for mine, ref in zip(*out):
+            np.testing.assert_array_equal(np.isnan(mine), np.isnan(ref))
+            np.testing.assert_allclose(mine, ref, rtol=RTOL, atol=0)  # infinities and NaN equal theirs
