@@ -25,13 +25,11 @@
 // start out visited.
 #include "device_utils.cuh"
 #include "gu_internal.h"
+#include "kernel_fit.h"
 
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
-#include <map>
-#include <mutex>
-#include <tuple>
 
 namespace gu {
 
@@ -607,40 +605,7 @@ static SbConfig sb_config(const DeviceGraph &g, int S, int threads)
     c.mode = S > 1 ? SB_CLUSTER : g.n <= SB_BYTES_MAX_N ? SB_BYTES : SB_CTA;
     c.smem = sb_smem_bytes(c.slice, S, c.mode == SB_BYTES);
     if (c.smem > SB_MAX_SMEM) return c;
-    // the occupancy calculation costs as much as a small launch: kept by shape
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, int, size_t>, int> known;
-    std::lock_guard<std::mutex> lk(mu);
-    const auto key = std::make_tuple(g.device, S, threads, c.smem);
-    const auto it = known.find(key);
-    if (it != known.end()) {
-        c.resident = it->second;
-        return c;
-    }
-    const void *kern = sb_kernel(c.mode);
-    GU_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SB_MAX_SMEM));
-    if (S > 1) {
-        GU_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)S;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)S);
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = c.smem;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&c.resident, kern, &cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            c.resident = 0;
-        }
-    } else {
-        GU_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.resident, kern, threads, c.smem));
-        c.resident *= g.sm_count;
-    }
-    if (known.size() > 4096) known.clear();
-    known[key] = c.resident;
+    c.resident = kernel_fit(g.device, sb_kernel(c.mode), threads, c.smem, SB_MAX_SMEM, S) * (S > 1 ? 1 : g.sm_count);
     return c;
 }
 
