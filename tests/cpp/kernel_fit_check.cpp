@@ -9,7 +9,7 @@
 
 #include "kernel_fit.h"
 
-static int calls = 0;
+static int device = 0, calls = 0;  // the stand-in's current device
 static std::map<std::pair<int, const void *>, int> consent;
 static std::map<const void *, int> resident;
 
@@ -54,6 +54,7 @@ int main()
     CHECK(gu::kernel_fit(0, &b, 512, 72000, 228352) == 3);
     CHECK((consent[{0, &b}] == 228352));
     // the same kernel and shape on another device: consent there too
+    device = 1;
     CHECK(gu::kernel_fit(1, &a, 512, 72000, 228352) == 2);
     CHECK((consent[{1, &a}] == 228352));
     // clusters apart from single CTAs
@@ -61,6 +62,7 @@ int main()
     CHECK(gu::kernel_fit(1, &a, 512, 72000, 228352, 8) == 208);
     // asked again: kept
     const int before = calls;
+    device = 0;
     CHECK(gu::kernel_fit(0, &b, 512, 72000, 228352) == 3);
     CHECK(gu::kernel_fit(1, &a, 512, 72000, 228352, 8) == 208);
     CHECK(calls == before);
