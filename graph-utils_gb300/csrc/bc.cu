@@ -33,6 +33,7 @@
 #include "device_utils.cuh"
 #include "fp64_int.cuh"
 #include "gu_internal.h"
+#include "kernel_fit.h"
 
 #include <algorithm>
 #include <climits>
@@ -1075,17 +1076,11 @@ void launch_bc(DeviceGraph &g, const int32_t *sources, int32_t k, const BcOption
     GU_CUDA_CHECK(cudaMemsetAsync(a.ctl, 0, BC_TIMELINE_OFF + BC_TIMELINE_BYTES, stream));
     const void *kern = W == 1 ? (const void *)bc_grid_kernel<1>
                        : W == 2 ? (const void *)bc_grid_kernel<2> : (const void *)bc_grid_kernel<4>;
-    const int ki = W == 1 ? 0 : W == 2 ? 1 : 2;
     const size_t dyn = std::max(sizeof(RowTile), (size_t)(BC_THREADS / 32) * (W == 1   ? sizeof(SumStage<1>)
                                                                               : W == 2 ? sizeof(SumStage<2>)
                                                                                        : sizeof(SumStage<4>)));
-    static int occupancy[3] = {-1, -1, -1};
-    int &blocks_per_sm = occupancy[ki];
-    if (blocks_per_sm < 0) {
-        GU_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-        GU_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, BC_THREADS, dyn));
-        if (blocks_per_sm < 1) throw gu_error(GU_ERR_INTERNAL, "bc kernel cannot be resident");
-    }
+    const int blocks_per_sm = kernel_fit(g.device, kern, BC_THREADS, dyn, dyn);
+    if (blocks_per_sm < 1) throw gu_error(GU_ERR_INTERNAL, "bc kernel cannot be resident");
     int nblocks = g.sm_count * blocks_per_sm;
     if (opt.max_blocks > 0 && nblocks > opt.max_blocks) nblocks = opt.max_blocks;
     dim3 grid(nblocks), block(BC_THREADS);

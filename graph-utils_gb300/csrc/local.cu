@@ -26,6 +26,7 @@
 // chain.
 #include "device_utils.cuh"
 #include "gu_internal.h"
+#include "kernel_fit.h"
 #include "recent.h"
 
 #include <algorithm>
@@ -424,16 +425,9 @@ bool launch_local_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t
                                              local_bfs_kernel<true, 16>, mesh_bfs_kernel<true>}};
     auto kern = kerns[rows][wi];
     auto smem_for = [&](int ring) { return mesh ? MESH_SMEM : ring * sizeof(int32_t) + RECENT_SLOTS * sizeof(uint16_t); };
-    static bool attr_set[2][4];
-    if (!attr_set[rows][wi]) {
-        GU_CUDA_CHECK(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem_for(LOCAL_WIDE_RING)));
-        attr_set[rows][wi] = true;
-    }
     const int ring = g.local_wide ? LOCAL_WIDE_RING : LOCAL_RING;
     const size_t smem = smem_for(ring);
-    int per_sm = 0;
-    GU_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)kern, LOCAL_THREADS, smem));
+    const int per_sm = kernel_fit(g.device, (const void *)kern, LOCAL_THREADS, smem, smem_for(LOCAL_WIDE_RING));
     if (per_sm < 1) throw gu_error(GU_ERR_INTERNAL, "per-source BFS kernel cannot be resident");
     int grid = g.sm_count * per_sm;
     if (grid > k) grid = k;
