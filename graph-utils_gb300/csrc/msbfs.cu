@@ -1814,12 +1814,12 @@ __host__ __device__ inline void ms_layout(char *ctl, char *p, size_t n, int W, M
 // the workspace, with barriers over its own CTAs only.  Items of different graphs and
 // sizes run side by side on different groups.
 //
-// With fewer items than half the grid's CTAs every item has its own group, sized by the
-// item's estimated work (queue_weight): with equal groups the largest graphs' items
-// bounded the launch while the small ones' groups stood idle (24 requests on R-MAT
-// 12-16 and DAGs of 65536 vertices: 1415 us, sized
-// 900 us).  With more items the
-// groups are equal and the counter balances them.
+// With fewer items than half the grid's CTAs, and graphs small enough for as many equal
+// groups, every item has its own group, sized by the item's estimated work
+// (queue_weight): with equal groups the largest graphs' items bounded the launch while
+// the small ones' groups stood idle (24 requests on R-MAT 12-16 and DAGs of 65536
+// vertices: 1415 us, sized 900 us).  Else the groups are equal and the counter balances
+// them.
 struct MqItem {
     const int32_t *R, *C, *RT, *CT;
     const int32_t *light, *mid, *wide, *heavy;
@@ -2088,44 +2088,54 @@ MsQueueLaunch msbfs_queue_plan(const std::vector<MsQueueRequest> &reqs, int sms,
     const int bps = L.W == 1 ? queue_blocks_per_sm<1>() : L.W == 2 ? queue_blocks_per_sm<2>() : queue_blocks_per_sm<4>();
     int blocks = sms * bps;
     if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
-    size_t data = 0;  // workspace slices, after the control regions
-    if (2 * L.items <= blocks) {
-        std::vector<double> w;
-        std::vector<size_t> n;
-        double sum = 0;
-        for (const MsQueueRequest &r : reqs)
-            for (int32_t off = 0; off < r.k; off += per_item) {
-                w.push_back(queue_weight(r, std::min(per_item, r.k - off)));
-                n.push_back((size_t)r.g->n);
-                sum += w.back();
-            }
-        int base = 0;
-        for (size_t i = 0; i < w.size(); ++i) {
-            const int size = 1 + (int)((double)(blocks - L.items) * (w[i] / sum));
-            L.groups.push_back({base, size, (int)i, data});
-            base += size;
-            data += ms_up256(ms_data_bytes(n[i], L.W));
+    // Where the slices of the groups' data start (after the control regions), and the
+    // bytes of the whole workspace.
+    auto lay_out = [](MsQueueLaunch &q, const std::vector<size_t> &slice) {
+        size_t at = q.groups.size() * WS_CONTROL_BYTES;
+        for (size_t i = 0; i < q.groups.size(); ++i) {
+            q.groups[i].data = at;
+            at += slice[i];
         }
-        L.grid = std::min(base, blocks);
-        L.groups.back().size -= base - L.grid;  // (a rounding of the shares upwards, if any)
-        L.taken = L.items;
-    } else {
-        // equal groups: about 16 K vertices of the largest graph per CTA, larger while
-        // there are fewer items than groups
-        int gs = (int)std::min<size_t>((maxn + 16383) / 16384, (size_t)blocks);
-        gs = std::max(1, std::min(std::max(gs, blocks / L.items), blocks));
-        const size_t slice = ms_up256(ms_data_bytes(maxn, L.W));
-        for (int i = 0; i < blocks / gs; ++i, data += slice) L.groups.push_back({i * gs, gs, -1, data});
-        L.grid = (int)L.groups.size() * gs;
-        L.taken = 0;
+        q.items_off = at;
+        q.groups_off = q.items_off + ms_up256(sizeof(MqItem) * (size_t)q.items);
+        q.cnt_off = q.groups_off + ms_up256(sizeof(MqGroup) * q.groups.size());
+        q.bytes = q.cnt_off + 256;
+    };
+    // equal groups: about 16 K vertices of the largest graph per CTA, larger while
+    // there are fewer items than groups
+    MsQueueLaunch equal = L;
+    int gs = (int)std::min<size_t>((maxn + 16383) / 16384, (size_t)blocks);
+    gs = std::max(1, std::min(std::max(gs, blocks / L.items), blocks));
+    for (int i = 0; i < blocks / gs; ++i) equal.groups.push_back({i * gs, gs, -1, 0});
+    equal.grid = (int)equal.groups.size() * gs;
+    equal.taken = 0;
+    lay_out(equal, std::vector<size_t>(equal.groups.size(), ms_up256(ms_data_bytes(maxn, L.W))));
+    if (2 * L.items > blocks) return equal;
+    // A group per item.  Every item then has a slice of its own, where the number of
+    // equal groups falls as the graphs grow: taken while it needs no more memory, which
+    // is also about where it is faster (R-MAT 20, 24 requests of 200 sources: 19.1 ms and
+    // 18.8 GB, equal groups 16.9 ms and 3.2 GB; R-MAT 18, 60 of 60: 6.2 and 4.7 ms;
+    // R-MAT 18, 24 of 200: 4.6 and 4.8).
+    std::vector<double> w;
+    std::vector<size_t> slice;
+    double sum = 0;
+    for (const MsQueueRequest &r : reqs)
+        for (int32_t off = 0; off < r.k; off += per_item) {
+            w.push_back(queue_weight(r, std::min(per_item, r.k - off)));
+            slice.push_back(ms_up256(ms_data_bytes((size_t)r.g->n, L.W)));
+            sum += w.back();
+        }
+    int base = 0;
+    for (size_t i = 0; i < w.size(); ++i) {
+        const int size = 1 + (int)((double)(blocks - L.items) * (w[i] / sum));
+        L.groups.push_back({base, size, (int)i, 0});
+        base += size;
     }
-    const size_t ctl = L.groups.size() * WS_CONTROL_BYTES;
-    for (MsQueueLaunch::Group &g : L.groups) g.data += ctl;
-    L.items_off = ctl + data;
-    L.groups_off = L.items_off + ms_up256(sizeof(MqItem) * (size_t)L.items);
-    L.cnt_off = L.groups_off + ms_up256(sizeof(MqGroup) * L.groups.size());
-    L.bytes = L.cnt_off + 256;
-    return L;
+    L.grid = std::min(base, blocks);
+    L.groups.back().size -= base - L.grid;  // (a rounding of the shares upwards, if any)
+    L.taken = L.items;
+    lay_out(L, slice);
+    return L.bytes <= equal.bytes ? L : equal;
 }
 
 MsQueueLaunch launch_msbfs_queue(const std::vector<MsQueueRequest> &reqs, Workspace &wsp, int sms, int max_blocks,

@@ -40,3 +40,34 @@ def test_items_and_groups(graphs, items, kmax):
             assert (got[:, hg.n:] == -7).all()
         if cnt is not None:
             np.testing.assert_array_equal(cnt.cpu().numpy(), (ref != gu.UNREACHABLE).sum(1))
+
+
+@pytest.fixture(scope="module")
+def trees():
+    """Two trees on a million vertices: a slice of workspace for 64 sources is 0.23 GB."""
+    n = 1 << 20
+    return [gu.Graph(gu.HostGraph.from_edges(n, (np.arange(1, n) - 1) // f, np.arange(1, n))) for f in (16, 50)]
+
+
+def test_workspace_on_large_graphs(trees):
+    """As many slices of workspace as equal groups take (four here), however many requests."""
+    srcs = torch.arange(7, 9, dtype=torch.int32, device="cuda")
+    reqs = [(trees[i % 2], srcs, None, torch.zeros(2, dtype=torch.int64, device="cuda")) for i in range(32)]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    gu.bfs_many(reqs)
+    assert free - torch.cuda.mem_get_info()[0] < 1.3e9
+    for g, _, _, cnt in reqs:
+        assert cnt.tolist() == [g.n, g.n]
+
+
+def test_server_admits_what_equal_groups_take(trees):
+    """Forty one-source requests on both graphs, merged into one launch or a few, within a
+    budget of four slices and the outputs."""
+    srv = gu.Server(hbm_budget_bytes=3 << 29, slots=1)
+    out = [np.zeros(1, np.int64) for _ in range(40)]
+    ids = [srv.submit(trees[i % 2], gu.QUERY_REACH, np.array([i], np.int32), out[i]) for i in range(40)]
+    for i, rid in enumerate(ids):
+        assert srv.wait(rid, 60.0) is not None
+        assert out[i][0] == trees[i % 2].n
+    srv.close()
