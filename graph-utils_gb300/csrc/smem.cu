@@ -153,13 +153,11 @@ __global__ void __launch_bounds__(SB_MAX_THREADS, 1) smem_bfs_kernel(SbArgs a)
         else __syncthreads();
     };
     int par = 0, n_td = 0, n_bu = 0, deepest = 0, err = 0;
+    // every CTA checks all sources: a call with a bad one is refused and writes nothing
+    bool bad = false;
+    for (int i = threadIdx.x; i < a.k; i += T) bad |= (unsigned)__ldg(a.sources + i) >= (unsigned)a.n;
     for (int si = cid; si < a.k; si += nclusters) {
         const int32_t src = __ldg(a.sources + si);
-        const bool bad = (unsigned)src >= (unsigned)a.n;
-        if (bad) {  // reported by the call; its row is left as it was
-            err = DEV_ERR_BAD_SOURCE;
-            continue;
-        }
         for (int i = threadIdx.x; i < words; i += T) {
             const uint32_t bit = (src >> 5) == i ? 1u << (src & 31) : 0u;
             cur[i] = bit;
@@ -168,7 +166,10 @@ __global__ void __launch_bounds__(SB_MAX_THREADS, 1) smem_bfs_kernel(SbArgs a)
         for (int i = threadIdx.x; i < (MODE == SB_BYTES ? 8 : 1) * words; i += T) nxt[i] = 0;
         for (int i = threadIdx.x; i < a.slice * 16; i += T) reinterpret_cast<uint32_t *>(lev)[i] = 0xFFFFFFFFu;
         const bool mine = src >= v0 && src < v0 + a.slice * 32;
-        __syncthreads();
+        if (__syncthreads_or(bad)) {  // (with a barrier that is there anyway; the same for every CTA)
+            err = DEV_ERR_BAD_SOURCE;
+            break;
+        }
         if (threadIdx.x == 0) {
             s_qn = mine ? 1 : 0;
             s_nbig = 0;

@@ -105,14 +105,13 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
     double *part = BACKWARD ? a.part + (size_t)blockIdx.x * n : nullptr;
     if (BACKWARD)
         for (int v = threadIdx.x; v < n; v += T) part[v] = 0.0;
-    int err = 0, deepest = 0;
-    for (int si = blockIdx.x; si < a.k; si += gridDim.x) {
-        const int32_t given = __ldg(a.sources + si);
-        if ((unsigned)given >= (unsigned)n) {
-            err = DEV_ERR_BAD_SOURCE;
-            continue;
-        }
-        const int src = __ldg(a.newid + given);
+    int deepest = 0;
+    // every CTA checks all sources: a call with a bad one is refused and writes nothing
+    bool bad = false;
+    for (int i = threadIdx.x; i < a.k; i += T) bad |= (unsigned)__ldg(a.sources + i) >= (unsigned)n;
+    const int err = __syncthreads_or(bad) ? (int)DEV_ERR_BAD_SOURCE : 0;
+    for (int si = blockIdx.x; si < a.k && !err; si += gridDim.x) {
+        const int src = __ldg(a.newid + __ldg(a.sources + si));
         for (int v = threadIdx.x; v < vpad; v += T) {
             val[v] = v == src ? 1ull : 0ull;
             lev[v] = v == src ? 0 : (uint16_t)SC_NONE;

@@ -129,3 +129,25 @@ def test_tuned_to_this_engine():
     assert "shared-memory" in {t["engine"] for t in trials}
     g.set_tuning({"engine": "shared-memory"})
     np.testing.assert_array_equal(rows(g, srcs), ref)
+
+
+@pytest.mark.parametrize("n,k", [(198, 198), (3000, 300), (9000, 3), (20000, 7), (70000, 2)])
+def test_refused_calls_write_nothing(n, k):
+    """A source out of range, first or last: no row and no count is written, of the good
+    sources neither (byte form, one CTA, clusters; BC and sigma too where they fit)."""
+    hg = hub_graph(n, 9 * n, seed=n)
+    g = gu.Graph(hg)
+    for at, bad in ((0, n), (k - 1, -1)):
+        srcs = gu.sources(n, k, seed=1)
+        srcs[at] = bad
+        s = torch.as_tensor(srcs, device="cuda")
+        out = torch.full((k, n), -7, dtype=torch.int32, device="cuda")
+        sig = torch.full((k, n), -7, dtype=torch.int64, device="cuda")
+        delta = torch.full((k, n), -7.0, dtype=torch.float64, device="cuda")
+        bc = torch.full((n,), -7.0, dtype=torch.float64, device="cuda")
+        for call in (lambda: g.bfs(s, out), lambda: g.sigma(s, sig, dist_dev=out), lambda: g.bc(s, bc, delta_dev=delta)):
+            with pytest.raises(gu.GuError) as e:
+                call()
+            assert e.value.status == 1
+        for t in (out, sig, delta, bc):
+            assert (t == -7).all()
