@@ -664,20 +664,30 @@ static SbConfig sb_choose(const DeviceGraph &g, int32_t k)
 bool smem_bfs_takes(const DeviceGraph &g, int32_t k) { return sb_choose(g, k).S > 0; }
 
 // Rows (dist) and / or counts (reach) of k sources; false if AUTO does not take this
-// engine here or a level does not fit 16 bits (the caller runs another engine).
+// engine here, its tables cannot be allocated or a level does not fit 16 bits (the caller
+// runs another engine).
 // Synchronises stream.
 bool launch_smem_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t *dist, int64_t ld,
                      unsigned long long *reach, int *max_level, cudaStream_t stream)
 {
     const SbConfig c = sb_choose(g, k);
     if (c.S == 0) return false;
-    if (!g.sb_status) GU_CUDA_CHECK(pinned_alloc(&g.sb_status, sizeof(SbStatus) * SB_MAX_CLUSTERS));
+    // an allocation that fails: the other engines run the search in the memory they have
+    auto got = [](cudaError_t e) {
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        GU_CUDA_CHECK(e);
+        return true;
+    };
+    if (!g.sb_status && !got(pinned_alloc(&g.sb_status, sizeof(SbStatus) * SB_MAX_CLUSTERS))) return false;
     const int pad_words = (int)(((int64_t)g.n + 31) / 32) + 4 * SB_MAX_CLUSTER;  // slices are multiples of four words
     const size_t head_bytes = (size_t)g.n * sizeof(int4);
     if (!g.sb_head) {
         void *p = nullptr;
         const size_t bytes = head_bytes + (size_t)pad_words * sizeof(uint32_t);
-        GU_CUDA_CHECK(dev_malloc(&p, bytes));
+        if (!got(dev_malloc(&p, bytes))) return false;
         g.extra_allocs.push_back(p);
         g.bytes += bytes;
         g.sb_head = p;

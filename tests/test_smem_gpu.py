@@ -3,6 +3,7 @@ its sizes: word, slice and cluster boundaries, the byte form's last size, one CT
 sixteen per source, wide and long searches.  Distances, counts and levels are
 integers and must equal the oracle's exactly; the batched engine (GU_AUTO_LOCAL=0)
 must give the same rows."""
+import ctypes
 import os
 
 import numpy as np
@@ -151,3 +152,39 @@ def test_refused_calls_write_nothing(n, k):
             assert e.value.status == 1
         for t in (out, sig, delta, bc):
             assert (t == -7).all()
+
+
+@pytest.mark.parametrize("after", [0, 1])
+@pytest.mark.parametrize("n", [900, 9000, 40000])
+def test_without_memory_for_its_tables(n, after):
+    """Its first (pinned) or second (device) allocation fails: the search runs on another
+    engine, as on these graphs before this engine was there; a bad source is still
+    refused, and the next call takes this engine."""
+    hg = hub_graph(n, 8 * n, seed=n + after)
+    srcs = gu.sources(n, 5, seed=2)
+    ref, _ = oracle.bfs_multi(hg.R, hg.C, n, srcs, nthreads=4)
+    L = gu.lib()
+    L.gu_debug_fail_allocations.argtypes = [ctypes.c_int64, ctypes.c_int64]
+    s = torch.as_tensor(srcs, device="cuda")
+    for what in ("bfs", "reach", "diameter", "bad source"):
+        g = gu.Graph(hg)
+        cnt = torch.full((5,), -1, dtype=torch.int64, device="cuda")
+        out = torch.full((5, n), -7, dtype=torch.int32, device="cuda")
+        try:
+            assert L.gu_debug_fail_allocations(after, 1) == gu.OK
+            if what == "bfs":
+                g.bfs(s, out)
+                np.testing.assert_array_equal(out.cpu().numpy(), ref)
+            elif what == "reach":
+                g.reach(s, cnt)
+                np.testing.assert_array_equal(cnt.cpu().numpy(), (ref != gu.UNREACHABLE).sum(1))
+            elif what == "diameter":
+                assert g.diameter(s) == ref[ref != gu.UNREACHABLE].max()
+            else:
+                with pytest.raises(gu.GuError) as e:
+                    g.bfs(torch.tensor([1, n], dtype=torch.int32, device="cuda"), out[:2])
+                assert e.value.status == 1
+        finally:
+            L.gu_debug_fail_allocations(0, 0)
+        np.testing.assert_array_equal(rows(g, srcs), ref)
+        assert g.level_profile() == []
