@@ -16,6 +16,7 @@
 #include "gu_internal.h"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <string>
 
@@ -44,8 +45,8 @@ struct TopoCtl {
     int nlevels, total;
     u64 pack[4];  // appended vertices of a level, (count << 38) | out-edges
     u64 ins[4];   // ... and their in-edges
-    int top;      // reach_kernel: highest level of the batch's sources, plus one
-    int pad2;
+    int top;      // reach_kernel: highest level of the batch's sources
+    int deep;     // topo_plan_kernel stopped at its level limit
 };
 constexpr int TOPO_PACK = 38;
 
@@ -63,6 +64,7 @@ struct TopoArgs {
     int2 *IR;
     TopoCtl *ctl;
     unsigned long long wait_ns;
+    int max_levels;  // an order of more is not completed
 };
 
 // All lanes of the warp call it; lanes with pred place their vertex (out-degree deg,
@@ -133,6 +135,10 @@ __global__ void __launch_bounds__(TOPO_THREADS, TOPO_MIN_BLOCKS) topo_plan_kerne
         const u64 pk = s_pack[level & 3];
         const long long le = ls + (long long)(pk >> TOPO_PACK);
         if (le == ls) break;
+        if (level == a.max_levels) {
+            if (rank == 0) ctl->deep = 1;
+            return;
+        }
         const long long enext = ebase + (long long)(pk & ((1ull << TOPO_PACK) - 1ull));
         const long long inext = ibase + (long long)s_pack[4 + (level & 3)];
         if (rank == 0) {
@@ -454,23 +460,30 @@ static void check_topo(const TopoCtl &c)
     if (c.err != 0) throw gu_error(GU_ERR_INTERNAL, "device reported error code " + std::to_string(c.err));
 }
 
-// Builds the graph's topological order once (synchronises st); false if the graph
-// has a cycle.  ws_bytes: workspace that the caller takes next (allocated at once).
-static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
+// Builds the graph's topological order once (synchronises st); false if the graph has a
+// cycle or its order more than max_levels levels.  Only a completed order is kept: what
+// is known of the others is their state.  ws_bytes: workspace that the caller takes next
+// (allocated at once).
+static bool ensure_topo(DeviceGraph &g, int max_levels, size_t ws_bytes, cudaStream_t st)
 {
     TopoPlan &t = g.topo;
-    if (t.state != TopoPlan::UNBUILT) return t.state == TopoPlan::ACYCLIC;
+    if (t.state == TopoPlan::CYCLIC || (t.state == TopoPlan::DEEP && max_levels <= REACH_MAX_LEVELS)) return false;
+    if (t.state == TopoPlan::ACYCLIC) return t.nlevels <= max_levels;
     const size_t n = (size_t)g.n, m = (size_t)g.m;
     char *ws = (char *)g.ws.get(std::max(ws_bytes, WS_CONTROL_BYTES + 3 * n * sizeof(int32_t)));
     const size_t ints = 2 * n + 2 * n + (n + 2) + (n + 1) + 2 * m;
-    int32_t *buf = nullptr;
-    const cudaError_t e = dev_malloc((void **)&buf, ints * sizeof(int32_t));
+    struct Buffer {
+        int32_t *p = nullptr;
+        ~Buffer()
+        {
+            if (p) cudaFree(p);
+        }
+    } buf;
+    const cudaError_t e = dev_malloc((void **)&buf.p, ints * sizeof(int32_t));
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         throw gu_error(GU_ERR_OUT_OF_MEMORY, "topological order allocation failed");
     }
-    g.extra_allocs.push_back(buf);
-    g.bytes += ints * sizeof(int32_t);
     TopoArgs a;
     a.R = g.R;
     a.C = g.C;
@@ -480,8 +493,8 @@ static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
     a.m = g.m;
     a.in = reinterpret_cast<int2 *>(ws + WS_CONTROL_BYTES);
     a.cnt = reinterpret_cast<int32_t *>(a.in + n);
-    a.IR = reinterpret_cast<int2 *>(buf);
-    a.order = buf + 2 * n;
+    a.IR = reinterpret_cast<int2 *>(buf.p);
+    a.order = buf.p + 2 * n;
     a.pos = a.order + n;
     a.lvl = a.pos + n;
     a.PR = a.lvl + n + 2;
@@ -489,6 +502,7 @@ static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
     a.IC = a.PC + m;
     a.ctl = reinterpret_cast<TopoCtl *>(ws);
     a.wait_ns = wait_limit_ns();
+    a.max_levels = max_levels;
     GU_CUDA_CHECK(cudaMemsetAsync(ws, 0, WS_CONTROL_BYTES, st));
     void *params[] = {&a};
     GU_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)topo_plan_kernel, dim3(g.sm_count), dim3(TOPO_THREADS), params, 0, st));
@@ -496,6 +510,11 @@ static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
     GU_CUDA_CHECK(cudaMemcpyAsync(&c, ws, sizeof(c), cudaMemcpyDeviceToHost, st));
     GU_CUDA_CHECK(cudaStreamSynchronize(st));
     check_topo(c);
+    t.state = c.deep ? TopoPlan::DEEP : c.total == g.n ? TopoPlan::ACYCLIC : TopoPlan::CYCLIC;
+    if (t.state != TopoPlan::ACYCLIC) return false;
+    g.extra_allocs.push_back(buf.p);
+    buf.p = nullptr;
+    g.bytes += ints * sizeof(int32_t);
     t.order = a.order;
     t.lvl = a.lvl;
     t.pos = a.pos;
@@ -504,8 +523,7 @@ static bool ensure_topo(DeviceGraph &g, size_t ws_bytes, cudaStream_t st)
     t.IR = reinterpret_cast<int32_t *>(a.IR);
     t.IC = a.IC;
     t.nlevels = c.nlevels;
-    t.state = c.total == g.n ? TopoPlan::ACYCLIC : TopoPlan::CYCLIC;
-    return t.state == TopoPlan::ACYCLIC;
+    return true;
 }
 
 // The closure on bit rows; false where it does not apply (a cycle, too many
@@ -524,7 +542,11 @@ static bool launch_closure(DeviceGraph &g, unsigned long long *counts, cudaStrea
         const int64_t nblocks = (chunks + fit - 1) / fit;
         block = (chunks + nblocks - 1) / nblocks * CLOSURE_CHUNK;
         const size_t need = WS_CONTROL_BYTES + n * (size_t)(block / 8);
-        if (!ensure_topo(g, need, st)) return false;
+        const bool known = g.topo.state == TopoPlan::CYCLIC;
+        if (!ensure_topo(g, INT_MAX, need, st)) {
+            if (!known) g.ws.release();  // sized for the rows: the search takes what it needs
+            return false;
+        }
         ws = (char *)g.ws.get(need);
     } catch (const gu_error &e) {
         if (e.code == GU_ERR_OUT_OF_MEMORY) return false;
@@ -567,7 +589,7 @@ bool launch_dag_reach(DeviceGraph &g, const int32_t *sources, int32_t k, unsigne
     if (g.topo.state == TopoPlan::UNBUILT && g.topo.asked++ == 0) return false;
     try {
         const size_t need = WS_CONTROL_BYTES + sizeof(u64) * (size_t)g.n * W;
-        if (!ensure_topo(g, need, st) || g.topo.nlevels > REACH_MAX_LEVELS) return false;
+        if (!ensure_topo(g, REACH_MAX_LEVELS, need, st)) return false;
         ws = (char *)g.ws.get(need);
     } catch (const gu_error &e) {
         if (e.code == GU_ERR_OUT_OF_MEMORY) return false;

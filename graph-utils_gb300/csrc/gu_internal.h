@@ -143,7 +143,8 @@ constexpr float MS_ALPHA = 2.f;
 // vertices by the length of their longest path to a sink, so every successor of
 // the vertex at position p sits at a position below p's level.
 struct TopoPlan {
-    enum State { UNBUILT, ACYCLIC, CYCLIC } state = UNBUILT;
+    // DEEP: more levels than reachable counts go by (dag.cu); the closure builds it all the same
+    enum State { UNBUILT, ACYCLIC, CYCLIC, DEEP } state = UNBUILT;
     int32_t *order = nullptr;  // [n] vertex at position p
     int32_t *lvl = nullptr;    // [nlevels + 1] first position of each level
     int32_t *PR = nullptr;     // [n + 1] out-edge offsets by position

@@ -124,3 +124,39 @@ def test_reach_on_deep_and_cyclic_graphs():
             cnt = torch.full((8,), -1, dtype=torch.int64, device="cuda")
             g.reach(s, cnt)
             np.testing.assert_array_equal(cnt.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("levels", [96, 97, 5000])
+def test_orders_that_are_not_used_are_not_kept(levels):
+    """Reachable counts go by orders of up to 96 levels.  A deeper one is not built for them,
+    nor anything kept of it or of a graph with a cycle; the closure still builds it, and
+    the counts are the same throughout."""
+    n = 20000
+    v = np.arange(n)
+    u = v[(v % levels != levels - 1) & (v < n - 1)]
+    chains = gu.HostGraph.from_edges(n, u, u + 1, symmetric=False)
+    ring = gu.HostGraph.from_edges(n, v, (v + 1) % n, symmetric=False)
+    order_bytes = 4 * (6 * n + 3 + 2 * (n - n // levels - 1))
+    s = torch.arange(0, n, 2501, dtype=torch.int32, device="cuda")
+    at = s.cpu().numpy()
+    to_end = np.minimum(levels - 1 - at % levels, n - 1 - at) + 1  # a chain's vertices from each source on
+    for hg, want in ((chains, to_end), (ring, np.full(len(at), n))):
+        g = gu.Graph(hg)
+        cnt = torch.full((len(at),), -1, dtype=torch.int64, device="cuda")
+
+        def counts_are_right():
+            g.reach(s, cnt)
+            np.testing.assert_array_equal(cnt.cpu().numpy(), want)
+
+        counts_are_right()
+        before = g.device_bytes()
+        for _ in range(3):
+            counts_are_right()
+        kept = g.device_bytes() - before  # and what the workspace grew by, at most 0.35 MB here
+        assert (kept >= order_bytes) == (hg is chains and levels <= 96)
+        sizes = torch.empty(n, dtype=torch.int64, device="cuda")
+        g.dag_reach(sizes)
+        np.testing.assert_array_equal(sizes.cpu().numpy()[at], want - 1)
+        if hg is ring:  # the search's workspace, not the closure's rows (50 MB)
+            assert g.device_bytes() - before < 10e6
+        counts_are_right()
