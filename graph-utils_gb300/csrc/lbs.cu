@@ -13,11 +13,10 @@
 //      and the verdict on the call (no negative count, total within int32 and within
 //      the result capacity, a result buffer when the total is positive); scans its
 //      counts in registers, writes its part of scanned, and each warp writes the
-//      owners of its 256 items' slots: lanes store their items' ids into a window of
-//      1024 slots in shared memory and the window leaves as one bulk copy.
-//   3. lbs_expand_rest: the slots of warps whose items own more than 4096 slots, listed
-//      by kernel 2 in pieces of 4096; persistent CTAs find each slot's owner among the
-//      256 items by binary search.  With no such warp it ends at once.
+//      owners of its 256 items' slots (lbs_fill: found by binary search among the items;
+//      short lists by way of shared memory and a bulk copy).
+//   3. lbs_expand_rest: the slots of warps whose items own many, listed by kernel 2 in
+//      pieces of 2048, a warp each.  With no such warp it ends at once.
 //   Kernels 2 and 3 are launched as programmatic dependents of their predecessor, so
 //   that their launch overlaps its tail.  The total and the verdict go to pinned host
 //   memory; the host waits once, at the end.
@@ -37,10 +36,15 @@ constexpr int LBS_WARPS = LBS_THREADS / 32;
 constexpr int LBS_ITEMS = 8;                          // consecutive counts per thread
 constexpr int LBS_TILE = LBS_THREADS * LBS_ITEMS;     // counts per tile
 constexpr int LBS_WARP_ITEMS = 32 * LBS_ITEMS;
-constexpr int LBS_WINDOW = 1024;                      // slots staged at once by a warp
-constexpr int LBS_LOCAL = 4096;                       // slots that a warp of kernel 2 writes itself; piece of kernel 3
-constexpr int LBS_BIG = 32;                           // count from which the warp fills an item's slots together
+constexpr int LBS_LOCAL = 4096;                       // slots that a warp of kernel 2 always writes itself
+constexpr int LBS_SHARE = 13;                         // ... or 2^-13 of the total, if that is more
+constexpr int LBS_PIECE = 2048;                       // slots of a piece of kernel 3
+constexpr int LBS_KEYS = LBS_WARP_ITEMS + 4;
+constexpr int LBS_SHORT = 4;                          // counts up to which a warp's lists are short
+constexpr int LBS_CROWD = 8;                          // lanes that may start in one bank then
+constexpr int LBS_STAGE = LBS_WARP_ITEMS * LBS_SHORT + 8;
 constexpr int LBS_RTHREADS = 256;                     // kernel 3
+constexpr int LBS_REST_CTAS = 5;                      // ... CTAs per SM
 constexpr int LBS_DIRECT_TILES = 4096;                // tile sums that every tile adds up itself
 
 struct LbsHead {  // device scratch
@@ -155,23 +159,103 @@ __device__ __forceinline__ void bulk_store(void *dst, const void *src, unsigned 
 }
 __device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
+// The items of a warp that own slots, in order, as keys: first slot (from the first of the
+// slots to be written on) << 8 | item's number among the 256.  A lane comes with eight
+// consecutive items: the first slots and whether it owns any.
+__device__ __forceinline__ void lbs_keys(uint32_t *key, const uint32_t (&slot)[LBS_ITEMS], const bool (&owns)[LBS_ITEMS])
+{
+    const int lane = lane_id();
+#pragma unroll
+    for (int j = lane; j < LBS_KEYS; j += 32) key[j] = UINT32_MAX;
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < LBS_ITEMS; ++j) n += owns[j];
+    int at = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL_MASK, at, o);
+        if (lane >= o) at += y;
+    }
+    at -= n;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < LBS_ITEMS; ++j)
+        if (owns[j]) key[at++] = slot[j] << 8 | (uint32_t)(LBS_ITEMS * lane + j);
+    __syncwarp();
+}
+
+// The owners of n slots from `lo` on, by the warp's keys; its items start with `first`.
+// 128 slots at a time, four per lane from a 16-byte boundary of result on: a binary
+// search finds the first one's owner, and the others' owners are among the next three
+// keys, since every one of them owns a slot.  Two such steps are in flight.
+__device__ __forceinline__ void lbs_fill(const uint32_t *key, int32_t first, uint32_t lo, int n, int32_t *__restrict__ result)
+{
+    int32_t *dst = result + (long long)lo;
+    const int skip = (int)(((uintptr_t)dst >> 2) & 3);  // elements from a 16-byte boundary to dst
+    for (int t0 = -skip; t0 < n; t0 += 256) {           // warp-uniform
+        int t[2], l[2];
+        uint32_t x[2];  // keys below it: items whose first slot is at or before t
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            t[u] = t0 + 128 * u + 4 * lane_id();
+            x[u] = (uint32_t)(max(t[u], 0) + 1) << 8;
+            l[u] = 0;
+        }
+#pragma unroll
+        for (int step = LBS_WARP_ITEMS / 2; step > 0; step >>= 1)
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (key[l[u] + step] < x[u]) l[u] += step;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t k0 = key[l[u]], k1 = key[l[u] + 1], k2 = key[l[u] + 2], k3 = key[l[u] + 3];
+            const uint32_t x1 = (uint32_t)(t[u] + 2) << 8, x2 = x1 + 256, x3 = x2 + 256;
+            int4 o;
+            o.x = (int)k0;
+            o.y = (int)(k1 < x1 ? k1 : k0);
+            o.z = (int)(k2 < x2 ? k2 : k1 < x2 ? k1 : k0);
+            o.w = (int)(k3 < x3 ? k3 : k2 < x3 ? k2 : k1 < x3 ? k1 : k0);
+            o.x = first + (o.x & 255);
+            o.y = first + (o.y & 255);
+            o.z = first + (o.z & 255);
+            o.w = first + (o.w & 255);
+            if (t[u] >= 0 && t[u] + 4 <= n) {
+                *reinterpret_cast<int4 *>(dst + t[u]) = o;
+            } else {
+                if (t[u] >= 0 && t[u] < n) dst[t[u]] = o.x;
+                if (t[u] + 1 >= 0 && t[u] + 1 < n) dst[t[u] + 1] = o.y;
+                if (t[u] + 2 >= 0 && t[u] + 2 < n) dst[t[u] + 2] = o.z;
+                if (t[u] + 3 >= 0 && t[u] + 3 < n) dst[t[u] + 3] = o.w;
+            }
+        }
+    }
+}
+
 // Pass 2 (see the head of the file).  summed: sums holds prefixes (lbs_scan_sums).
-// Degree array of a 2048 x 2048 grid (N = 4.2 M, 15.9 M slots, 97 MB): the three
-// kernels take 30 us on the device, 0.48 of measured HBM; with the owners found by marks
-// and a running maximum over merge-path tiles, in a kernel of its own, they took 45 us
-// (the shared-memory pipe was the bound: three passes over every slot's mark; here a
-// slot is stored once and the window is read by the copy engine).  The call: 71 -> 44
-// us, also for want of two copies into pageable memory.  Counts of 0.1-density 1 .. 39:
-// device 44.5 -> 39 us; heavy-tailed counts (exponent 1.4): 43.6 -> 46 us, call 71 -> 60.
-// Two CTAs per SM: three, with 42 registers, took 32.5 us, six of 256 threads 33.1.
-// Filling items together from counts of 8 up: 46 and 54 us on the last two.
-__global__ void __launch_bounds__(LBS_THREADS, 2) lbs_scan_expand(const int32_t *__restrict__ counts, int32_t N, int32_t ntiles,
+//
+// A warp's slots.  Lists of up to four (a mesh's degrees): every lane stores its items'
+// ids to shared memory, and the warp's slots leave as one bulk copy.  Longer lists, and
+// equal ones whose lanes would store into the same few banks: by search.  Storing longer
+// lists item by item left most lanes idle and met conflicts of up to 32 lanes, and the
+// warps above 4096 slots were left to a kernel 3 of two CTAs per SM.  Calls in us, that
+// form / this one / with the owners found by marks and a running maximum over merge-path
+// tiles in a kernel of its own, N = 2^22: degrees of a grid with 5 % of its edges deleted
+// 43 / 41 / 75; all counts 4: 99 / 49 / 90, 16: 267 / 77 / 152, 20: 829 / 89 / 173; counts
+// 0 .. 8 60 / 50 / 89, 0 .. 32 532 / 80 / 154; heavy-tailed (exponent 1.4, mean 2.8) 60 /
+// 54 / 79; N = 262144, counts 0 .. 400 249 / 85 / 120.
+//
+// On the grid the three kernels take about 28 us, 0.5 of measured HBM: without the stores
+// of the owners they take as long, so the bound is the tiles' dependent chain (counts,
+// sums, scan, slots).  Three CTAs per SM: two 41.8 us a call, three 40.5; lists of up to
+// three as short ones 46.8.  What a warp writes itself: 4096 slots or 2^-13 of the total;
+// with 2^-11 heavy tails wait for single warps (mean 56, N = 2^22: 119 us, 96).
+__global__ void __launch_bounds__(LBS_THREADS, 3) lbs_scan_expand(const int32_t *__restrict__ counts, int32_t N, int32_t ntiles,
                                                               const long long *__restrict__ sums, int summed,
                                                               int32_t *__restrict__ scanned, LbsHead *head,
                                                               LbsReport *report, int32_t *total_out, long long capacity,
                                                               int32_t *__restrict__ result, int2 *__restrict__ list)
 {
-    extern __shared__ __align__(16) int32_t s_stage[];  // [LBS_WARPS][LBS_WINDOW]
+    extern __shared__ __align__(16) int32_t s_stage[];  // [LBS_WARPS][LBS_STAGE]
     __shared__ long long s_part[LBS_WARPS], s_all[LBS_WARPS], s_warp[LBS_WARPS];
     griddep_launch_dependents();
     const int lane = lane_id(), warp = warp_in_block(), t = blockIdx.x;
@@ -251,45 +335,37 @@ __global__ void __launch_bounds__(LBS_THREADS, 2) lbs_scan_expand(const int32_t 
     const long long R = __shfl_sync(FULL_MASK, inc, 31);
     if (R == 0) return;  // warp-uniform, no barrier below
     const int32_t first = (int32_t)((long long)t * LBS_TILE + warp * LBS_WARP_ITEMS);
-    if (R > LBS_LOCAL) {
-        const unsigned n = (unsigned)((R + LBS_LOCAL - 1) / LBS_LOCAL);
+    if (R > max((long long)LBS_LOCAL, total >> LBS_SHARE)) {
+        const unsigned n = (unsigned)((R + LBS_PIECE - 1) / LBS_PIECE);
         unsigned pos = 0;
         if (lane == 0) pos = atomicAdd(&head->pieces, n);
         pos = __shfl_sync(FULL_MASK, pos, 0);
-        for (unsigned j = lane; j < n; j += 32) list[pos + j] = make_int2(first, (int)(P + (long long)j * LBS_LOCAL));
+        for (unsigned j = lane; j < n; j += 32) list[pos + j] = make_int2(first, (int)(P + (long long)j * LBS_PIECE));
         return;
     }
-    int32_t *stage = s_stage + warp * LBS_WINDOW;
-    const int ra = (int)(((uintptr_t)result >> 2) & 3);  // result's element offset from a 16-byte boundary
-    const long long s1 = P + R;
-    // windows start at 16-byte boundaries of result (the first one at or below P)
-    for (long long a = P - ((P + ra) & 3); a < s1; a += LBS_WINDOW) {
-        const uint32_t lo = (uint32_t)max(a, P), hi = (uint32_t)min(a + LBS_WINDOW, s1);
-        const int32_t base = (int32_t)a;  // (a >= -3; differences to it stay small)
+    int32_t *stage = s_stage + warp * LBS_STAGE;
+    int most = 0;
 #pragma unroll
-        for (int j = 0; j < LBS_ITEMS; ++j) {
-            const uint32_t b = max(off[j], lo), e = min(off[j] + (uint32_t)c[j], hi);
-            const bool big = c[j] >= LBS_BIG && b < e;
-            const int cnt = big || e <= b ? 0 : (int)(e - b);
-            int32_t *p0 = stage + ((int32_t)b - base);
+    for (int j = 0; j < LBS_ITEMS; ++j) {
+        most = max(most, c[j]);
+        off[j] -= (uint32_t)P;
+    }
+    int32_t *dst = result + P;
+    // Short lists: every lane stores its items' ids to the warp's slots in shared memory,
+    // which leave as one bulk copy -- unless equal lists put the lanes' stores into the
+    // same few banks (lists of four: 32 lanes in one).
+    if (!__any_sync(FULL_MASK, most > LBS_SHORT) &&
+        !__any_sync(FULL_MASK, __popc(__match_any_sync(FULL_MASK, off[0] & 31u)) > LBS_CROWD)) {
+        const int x0 = (int)(((uintptr_t)dst >> 2) & 3), x1 = x0 + (int)R;  // from dst's 16-byte boundary on
+        const int m0 = (x0 + 3) & ~3, m1 = x1 & ~3;                        // ... the whole 16-byte pieces
 #pragma unroll
-            for (int q = 0; q < 4; ++q)  // short counts without a loop
-                if (q < cnt) p0[q] = (int32_t)(i0 + j);
-            for (int q = 4; q < cnt; ++q) p0[q] = (int32_t)(i0 + j);
-            unsigned todo = __ballot_sync(FULL_MASK, big);
-            while (todo) {
-                const int l = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const uint32_t bb = __shfl_sync(FULL_MASK, b, l), ee = __shfl_sync(FULL_MASK, e, l);
-                const int32_t id = first + l * LBS_ITEMS + j;
-                for (uint32_t p = bb + lane; p < ee; p += 32) stage[(int32_t)p - base] = id;
-            }
-        }
+        for (int j = 0; j < LBS_ITEMS; ++j)
+#pragma unroll
+            for (int q = 0; q < LBS_SHORT; ++q)
+                if (q < c[j]) stage[x0 + (int)off[j] + q] = (int32_t)(i0 + j);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stores above, before the copy engine reads
         __syncwarp();
-        const int x0 = (int)(lo - (uint32_t)base), x1 = (int)(hi - (uint32_t)base);  // the window's slots, by position
-        const int m0 = (x0 + 3) & ~3, m1 = x1 & ~3;           // ... in whole 16-byte pieces
-        int32_t *dst = result + a;
+        dst -= x0;
         if (m1 > m0 && lane == 0) bulk_store(dst + m0, stage + m0, (unsigned)(m1 - m0) * 4u);
         if (lane < 4) {  // the ends
             const int x = x0 + lane;
@@ -299,51 +375,50 @@ __global__ void __launch_bounds__(LBS_THREADS, 2) lbs_scan_expand(const int32_t 
             if (x < x1) dst[x] = stage[x];
         }
         if (m1 > m0 && lane == 0) bulk_store_wait_read();
-        __syncwarp();
+        return;
     }
+    bool owns[LBS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < LBS_ITEMS; ++j) owns[j] = c[j] > 0;
+    uint32_t *key = reinterpret_cast<uint32_t *>(stage);
+    lbs_keys(key, off, owns);
+    lbs_fill(key, first, (uint32_t)P, (int)R, result);
 }
 
-// The listed pieces: (first item of a warp's 256, first slot).
+// The listed pieces, a warp each: (first item of a warp's 256, first slot).
 __global__ void __launch_bounds__(LBS_RTHREADS) lbs_expand_rest(const int32_t *__restrict__ scanned, int32_t N,
                                                                const LbsHead *head, const int2 *__restrict__ list,
                                                                int32_t *__restrict__ result)
 {
-    __shared__ uint32_t s_off[LBS_WARP_ITEMS + 1];
+    __shared__ uint32_t s_key[LBS_RTHREADS / 32][LBS_KEYS];
     griddep_wait();
-    const unsigned pieces = head->pieces;
-    const int ra = (int)(((uintptr_t)result >> 2) & 3);
-    for (unsigned x = blockIdx.x; x < pieces; x += gridDim.x) {
+    const unsigned pieces = head->pieces, nw = gridDim.x * (LBS_RTHREADS / 32);
+    const uint32_t total = (uint32_t)head->total;
+    uint32_t *key = s_key[warp_in_block()];
+    for (unsigned x = blockIdx.x * (LBS_RTHREADS / 32) + warp_in_block(); x < pieces; x += nw) {  // warp-uniform
         const int2 pc = __ldcg(list + x);
-        const int32_t first = pc.x, items = min(LBS_WARP_ITEMS, N - first);
-        for (int i = threadIdx.x; i <= items; i += LBS_RTHREADS)
-            s_off[i] = first + i < N ? (uint32_t)__ldcg(scanned + first + i) : (uint32_t)head->total;
-        __syncthreads();
-        const uint32_t lo = (uint32_t)pc.y, hi = min(lo + LBS_LOCAL, s_off[items]);
-        const long long a = (long long)lo - ((lo + ra) & 3);
-        for (long long p0 = a + 4 * threadIdx.x; p0 < hi; p0 += 4 * LBS_RTHREADS) {
-            const uint32_t p = (uint32_t)max(p0, (long long)lo);
-            int l = 0, h = items - 1;  // the last item whose first slot is at or before p
-            while (l < h) {
-                const int mid = (l + h + 1) >> 1;
-                if (s_off[mid] <= p) l = mid;
-                else h = mid - 1;
-            }
-            int32_t o[4];
+        const int32_t first = pc.x;
+        const uint32_t lo = (uint32_t)pc.y;
+        __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t q = (uint32_t)max(p0 + j, (long long)lo);
-                while (l + 1 < items && s_off[l + 1] <= q) ++l;
-                o[j] = first + l;
-            }
-            if (p0 >= (long long)lo && p0 + 4 <= (long long)hi) {
-                *reinterpret_cast<int4 *>(result + p0) = make_int4(o[0], o[1], o[2], o[3]);
-            } else {
+        for (int i = lane_id(); i <= LBS_WARP_ITEMS; i += 32)
+            key[i] = i < N - first ? (uint32_t)__ldcg(scanned + first + i) : total;
+        __syncwarp();
+        const uint32_t hi = min(lo + LBS_PIECE, key[LBS_WARP_ITEMS]);
+        uint32_t slot[LBS_ITEMS + 1];
+        bool owns[LBS_ITEMS];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (p0 + j >= (long long)lo && p0 + j < (long long)hi) result[p0 + j] = o[j];
-            }
+        for (int j = 0; j <= LBS_ITEMS; ++j) slot[j] = key[LBS_ITEMS * lane_id() + j];
+        uint32_t from[LBS_ITEMS];
+#pragma unroll
+        for (int j = 0; j < LBS_ITEMS; ++j) {  // the item's slots within the piece
+            const uint32_t a = max(slot[j], lo);
+            owns[j] = a < min(slot[j + 1], hi);
+            from[j] = a - lo;
         }
-        __syncthreads();
+        __syncwarp();
+        lbs_keys(key, from, owns);
+        lbs_fill(key, first, lo, (int)(hi - lo), result);
     }
 }
 
@@ -355,15 +430,15 @@ __global__ void race_and_resolve_kernel(const int32_t *__restrict__ pred, int32_
     winner[i] = race_and_resolve_warp(pred[i] != 0);
 }
 
-// Scratch: the head, one sum per tile and the total, kernel 3's list (a warp with more
-// than LBS_LOCAL slots lists at most twice its slots / LBS_LOCAL pieces).
+// Scratch: the head, one sum per tile and the total, kernel 3's list (a warp with R >
+// LBS_LOCAL slots lists at most R / LBS_PIECE + 1 pieces, less than 3 R / LBS_LOCAL).
 constexpr size_t LBS_HEAD = 64;
 size_t lbs_scratch_bytes(int32_t N, int64_t result_capacity)
 {
     const long long n = N > 0 ? N : 0;
     const size_t ntiles = (size_t)((n + LBS_TILE - 1) / LBS_TILE);
     const long long cap = result_capacity < 0 ? 0 : (result_capacity > INT32_MAX ? INT32_MAX : result_capacity);
-    return LBS_HEAD + (ntiles + 1) * sizeof(long long) + (2 * (size_t)(cap / LBS_LOCAL) + 2) * sizeof(int2);
+    return LBS_HEAD + (ntiles + 1) * sizeof(long long) + (3 * (size_t)(cap / LBS_LOCAL) + 4) * sizeof(int2);
 }
 
 // Device time of the last call on each device: from before the flags are
@@ -416,7 +491,7 @@ void launch_lbs(const int32_t *counts, int32_t N, int32_t *scanned, int32_t *res
             cfg.blockDim = dim3(1024);
             GU_CUDA_CHECK(cudaLaunchKernelEx(&cfg, lbs_scan_sums, sums, ntiles));
         }
-        constexpr size_t stage_bytes = sizeof(int32_t) * LBS_WARPS * LBS_WINDOW;
+        constexpr size_t stage_bytes = sizeof(int32_t) * LBS_WARPS * LBS_STAGE;
         static bool attr[128];
         if (!attr[dev]) {
             GU_CUDA_CHECK(cudaFuncSetAttribute((const void *)lbs_scan_expand, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -432,7 +507,7 @@ void launch_lbs(const int32_t *counts, int32_t N, int32_t *scanned, int32_t *res
         int &sms = sms_of[dev];
         if (!sms) GU_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         cfg.dynamicSmemBytes = 0;
-        cfg.gridDim = dim3((unsigned)sms * 2);
+        cfg.gridDim = dim3((unsigned)sms * LBS_REST_CTAS);
         cfg.blockDim = dim3(LBS_RTHREADS);
         GU_CUDA_CHECK(cudaLaunchKernelEx(&cfg, lbs_expand_rest, (const int32_t *)scanned, N, (const LbsHead *)head,
                                          (const int2 *)list, result));

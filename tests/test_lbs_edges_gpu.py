@@ -46,6 +46,36 @@ def test_tiles_with_mixed_counts(n):
         check(heavy, *offs)
 
 
+@pytest.mark.parametrize("r_off", range(8))
+def test_short_lists_searches_and_pieces(r_off):
+    """The forms that a warp's slots are written in, at every alignment of the result and
+    next to each other: short lists (counts up to 4) with few and with many lanes in a
+    bank, items without slots between the others, searches up to 4096 slots, and pieces
+    of 2048 beyond, which start and end inside items."""
+    rng = np.random.default_rng(r_off)
+    for n in (256, 300, 513):
+        for c in (1, 2, 3, 4, 5, 8, 15, 16, 17, 40):
+            check(np.full(n, c), r_off)
+        for p in (0.02, 0.3):  # few items own slots
+            check(np.where(rng.random(n) < p, rng.integers(1, 5, n), 0), r_off)
+            check(np.where(rng.random(n) < p, rng.integers(1, 90, n), 0), r_off)
+    for last in (15, 16, 17, 2047, 2048, 2049, 4111, 6001):  # 4080 slots and the last item's
+        check([16] * 255 + [last], r_off)
+        check([last] + [16] * 255 + [0, 0, 3], r_off)
+    check(np.concatenate([rng.integers(0, 5, 256), rng.integers(0, 40, 256), rng.integers(100, 900, 256), [4] * 256,
+                          [0] * 256, [70000], rng.integers(0, 3, 700)]), r_off)
+
+
+def test_warps_write_more_of_a_large_total():
+    """Beyond 4096 slots a warp writes 2^-13 of the total itself: 5500 of 46 M, next to
+    warps with more."""
+    rng = np.random.default_rng(1)
+    counts = np.full(2_100_000, 21)
+    counts[rng.integers(0, len(counts), 50)] = 3000
+    counts[::7] += 1
+    check(counts, 1)
+
+
 def test_more_tiles_than_are_added_directly():
     rng = np.random.default_rng(2)
     n = 4096 * 4097 + 11
