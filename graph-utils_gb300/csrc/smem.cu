@@ -20,9 +20,9 @@
 //              first, until one is in the frontier
 // Then the owner records the level of the new vertices, queues them, counts them
 // and their out-edges; after a cluster barrier every CTA gathers all slices' new
-// bits as the next frontier.  Direction as in the batched engine (after Beamer,
-// Asanovic, Patterson, SC'12).  Vertices without in-edges are never scanned: they
-// start out visited.
+// bits as the next frontier.  Direction after Beamer, Asanovic, Patterson (SC'12), by the
+// work that each would be.  Vertices without in-edges are never scanned: they start out
+// visited.
 #include "device_utils.cuh"
 #include "gu_internal.h"
 #include "kernel_fit.h"
@@ -71,6 +71,7 @@ struct SbArgs {
     const int4 *__restrict__ head;      // [n] first four in-neighbours (-1: none)
     const uint32_t *__restrict__ none;  // bitmap of the vertices without in-edges, padded with ones
     int slice;  // bitmap words per CTA of a cluster
+    int32_t live;  // vertices with in-edges
     float alpha, beta;
     SbStatus *status;  // [clusters], pinned host memory
 };
@@ -189,8 +190,13 @@ __global__ void __launch_bounds__(SB_MAX_THREADS, 1) smem_bfs_kernel(SbArgs a)
             if (level > 1) {
                 // (32-bit floats: FP64 runs at two lanes a cycle per SM on this part, and a
                 // few such instructions in every warp cost more than the rest of the level end)
-                // A frontier of few edges is one round of loads top-down, whatever the graph.
-                if (!bu) bu = wide || ((float)fe * a.alpha > (float)a.m && fe > (long long)(4 * S) * T);
+                // Bottom-up, each of the vertices not reached tries its in-neighbours until one
+                // is in the frontier, m / fe of them at random: fewer than the frontier's fe
+                // out-edges if fe^2 > alpha x vertices left x m.  A frontier of few edges is
+                // one round of loads top-down, whatever the graph.
+                if (!bu)
+                    bu = wide || ((float)fe * (float)fe > a.alpha * (float)(a.live - reached) * (float)a.m &&
+                                  fe > (long long)(4 * S) * T);
                 else bu = (float)nf * a.beta > (float)a.n || nf > SB_QCAP;
             }
             if (threadIdx.x == 0) {
@@ -462,9 +468,11 @@ __global__ void __launch_bounds__(SB_MAX_THREADS, 1) smem_bfs_kernel(SbArgs a)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) edges += __shfl_xor_sync(FULL_MASK, edges, o);
             found_n = __reduce_add_sync(FULL_MASK, found_n);
-            if (lane == 0 && found_n) {
-                atomicAdd(&s_cnt[par].vertices, found_n);
-                atomicAdd(reinterpret_cast<unsigned long long *>(&s_cnt[par].edges), (unsigned long long)edges);
+            // (vertices are counted by bitmap word, their edges by place in the queue: a warp
+            // may have either without the other)
+            if (lane == 0) {
+                if (found_n) atomicAdd(&s_cnt[par].vertices, found_n);
+                if (edges) atomicAdd(reinterpret_cast<unsigned long long *>(&s_cnt[par].edges), (unsigned long long)edges);
             }
             __syncthreads();
             if (threadIdx.x == 0) s_cnt[par].overflow = !bu && s_qn > SB_QCAP;
@@ -711,7 +719,14 @@ bool launch_smem_bfs(DeviceGraph &g, const int32_t *sources, int32_t k, int32_t 
     a.head = static_cast<const int4 *>(g.sb_head);
     a.none = reinterpret_cast<const uint32_t *>(static_cast<const char *>(g.sb_head) + head_bytes);
     a.slice = c.slice;
-    a.alpha = 8.f;
+    a.live = g.nlight + g.nmid + g.nwide + g.nheavy;
+    // The first in-neighbours are the hubs, so a skewed graph needs fewer tries.  Call times
+    // in us, alpha 0.4 / 0.55 / 0.7 / 1: R-MAT 14 k = 150 74 / 77 / 79 / 80, R-MAT 18 (ef 10)
+    // k = 4 90 / 90 / 104 / 106, R-MAT 15 k = 120 91 / 92 / 92 / 110; ER 100000 (24 entries a
+    // vertex) k = 8 105 / 98 / 86 / 86, k = 20 152 / 146 / 137 / 119.  (Frontier edges x 8 >
+    // m, the batched engine's form of the rule: ER 2000, k = 64 42, R-MAT 14 k = 150 73, but
+    // ER 100000, k = 20 146 and ER 8000 with 1000 entries a vertex, k = 1024 1758, 280 now.)
+    a.alpha = (double)g.max_in_degree * a.live > 8.0 * (double)g.m ? 0.5f : 1.f;
     a.beta = 24.f;
     a.status = static_cast<SbStatus *>(g.sb_status);
     const int nclusters = std::min(std::min(k, c.resident), SB_MAX_CLUSTERS);

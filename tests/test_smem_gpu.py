@@ -188,3 +188,23 @@ def test_without_memory_for_its_tables(n, after):
             L.gu_debug_fail_allocations(0, 0)
         np.testing.assert_array_equal(rows(g, srcs), ref)
         assert g.level_profile() == []
+
+
+def test_direction_counts_all_frontier_edges():
+    """1024 neighbours of the source, in the first words of the bitmap, with 40 out-edges
+    each: their edges are summed by other warps than find them, and all 40960 count.  The
+    second level is then searched bottom-up (40960^2 against 6975 vertices left x 200000
+    edges), and so is the third; with part of the edges the second would be top-down, as
+    the first and the last are, which find one and twenty vertices' neighbours."""
+    rng = np.random.default_rng(4)
+    n, mid, end = 16000, 1025, 8000
+    u = np.concatenate([np.zeros(1024, np.int64), np.repeat(np.arange(1, mid), 40), rng.integers(mid, end, 158000)])
+    v = np.concatenate([np.arange(1, mid), rng.integers(mid, end, 40960), rng.integers(mid, end, 158000)])
+    order = np.argsort(u, kind="stable")  # parallel edges stay: the counts are exact
+    R = np.concatenate([[0], np.cumsum(np.bincount(u, minlength=n))])
+    hg = gu.HostGraph(R, v[order], n, directed=True)
+    g = gu.Graph(hg)
+    got = rows(g, [0])
+    td, bu, ml = g.last_launch()[1:]
+    np.testing.assert_array_equal(got, oracle.bfs_multi(hg.R, hg.C, n, [0])[0])
+    assert g.level_profile() == [] and (td, bu, ml) == (2, 2, 3)
