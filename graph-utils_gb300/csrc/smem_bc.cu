@@ -34,12 +34,11 @@
 #include "device_utils.cuh"
 #include "fp64_int.cuh"
 #include "gu_internal.h"
+#include "kernel_fit.h"
 
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
-#include <map>
-#include <mutex>
 #include <vector>
 
 namespace gu {
@@ -90,7 +89,8 @@ __device__ __forceinline__ void shared_add_u64(u64 *p, u64 x)
     if (hi) atomicAdd(q + 1, hi);
 }
 
-template <bool BACKWARD>
+// ROWS: per-source rows are written (always without BACKWARD).
+template <bool BACKWARD, bool ROWS>
 __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
 {
     extern __shared__ __align__(16) u64 sc_mem[];
@@ -105,13 +105,22 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
     double *part = BACKWARD ? a.part + (size_t)blockIdx.x * n : nullptr;
     if (BACKWARD)
         for (int v = threadIdx.x; v < n; v += T) part[v] = 0.0;
-    int deepest = 0;
-    // every CTA checks all sources: a call with a bad one is refused and writes nothing
-    bool bad = false;
-    for (int i = threadIdx.x; i < a.k; i += T) bad |= (unsigned)__ldg(a.sources + i) >= (unsigned)n;
-    const int err = __syncthreads_or(bad) ? (int)DEV_ERR_BAD_SOURCE : 0;
-    for (int si = blockIdx.x; si < a.k && !err; si += gridDim.x) {
-        const int src = __ldg(a.newid + __ldg(a.sources + si));
+    int err = 0, deepest = 0;
+    // A call with a source out of range is refused and writes nothing: bc is written by the
+    // next kernel, but rows source by source, so every CTA looks at all sources first.
+    bool refused = false;
+    if (ROWS) {
+        for (int i = threadIdx.x; i < a.k; i += T) refused |= (unsigned)__ldg(a.sources + i) >= (unsigned)n;
+        refused = __syncthreads_or(refused);
+        if (refused) err = DEV_ERR_BAD_SOURCE;
+    }
+    for (int si = blockIdx.x; si < a.k && !refused; si += gridDim.x) {
+        const int32_t given = __ldg(a.sources + si);
+        if ((unsigned)given >= (unsigned)n) {
+            err = DEV_ERR_BAD_SOURCE;
+            continue;
+        }
+        const int src = __ldg(a.newid + given);
         for (int v = threadIdx.x; v < vpad; v += T) {
             val[v] = v == src ? 1ull : 0ull;
             lev[v] = v == src ? 0 : (uint16_t)SC_NONE;
@@ -203,14 +212,14 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
         }
         const int L = level - 1;  // the deepest level; level l is ord[lstart[l] .. lstart[l + 1])
         deepest = max(deepest, L);
-        if (a.dist_rows || a.sigma_rows)
+        if (ROWS && (a.dist_rows || a.sigma_rows))
             for (int v = threadIdx.x; v < n; v += T) {
                 const int x = __ldg(a.newid + v);
                 if (a.dist_rows) __stcs(a.dist_rows + (int64_t)si * a.ld + v, lev[x] == SC_NONE ? INT_MAX : (int32_t)lev[x]);
                 if (a.sigma_rows) __stcs(a.sigma_rows + (int64_t)si * a.ld + v, val[x]);
             }
         if (BACKWARD) {
-            double *drow = a.delta_rows ? a.delta_rows + (int64_t)si * a.ld : nullptr;
+            double *drow = ROWS && a.delta_rows ? a.delta_rows + (int64_t)si * a.ld : nullptr;
             if (drow)  // 0 at the source, where unreached and on the last level
                 for (int v = threadIdx.x; v < n; v += T) drow[v] = 0.0;
             __syncthreads();
@@ -433,7 +442,8 @@ void launch_smem_bc(DeviceGraph &g, const int32_t *sources, int32_t k, double *b
 {
     ensure_renumbered(g, stream);
     const bool back = bc != nullptr;
-    const void *kern = back ? (const void *)smem_bc_kernel<true> : (const void *)smem_bc_kernel<false>;
+    const void *kern = !back        ? (const void *)smem_bc_kernel<false, true>
+                       : delta_rows ? (const void *)smem_bc_kernel<true, true> : (const void *)smem_bc_kernel<true, false>;
     const size_t smem = sc_smem_bytes(g.n);
     // Threads per source: wide where a source has an SM to itself (by shared memory, or
     // because there are few), narrow where several share one.  Call times with 128 / 256 /
@@ -444,19 +454,7 @@ void launch_smem_bc(DeviceGraph &g, const int32_t *sources, int32_t k, double *b
     const int threads = g.n > 4096   ? 1024
                         : g.n > 1024 ? (k <= sms ? 1024 : 512)
                                      : (k <= 2 * sms ? 512 : k <= 4 * sms ? 256 : 128);
-    int per_sm = 0;
-    {
-        static std::mutex mu;
-        static std::map<std::pair<int, size_t>, int> known;  // CTAs per SM by (device, kernel) and shared memory
-        std::lock_guard<std::mutex> lk(mu);
-        int &p = known[std::make_pair((2 * g.device + back) * 2048 + threads, smem)];
-        if (p == 0) {
-            GU_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)sc_smem_bytes(SC_MAX_N)));
-            GU_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, kern, threads, smem));
-        }
-        per_sm = p;
-    }
+    const int per_sm = kernel_fit(g.device, kern, threads, smem, sc_smem_bytes(SC_MAX_N));
     if (per_sm < 1) throw gu_error(GU_ERR_INTERNAL, "shared-memory BC kernel cannot be resident");
     const int grid = std::min(k, g.sm_count * per_sm);
     if (!g.sc_report) GU_CUDA_CHECK(pinned_alloc(&g.sc_report, sizeof(u64) * 4096));
