@@ -178,7 +178,7 @@ struct DeviceGraph {
     void *sb_status = nullptr;  // shared-memory engine: its clusters' reports (pinned)
     int sb_clusters = 0;        // ... of the last launch
     void *sc_graph = nullptr;   // shared-memory BC engine: the graph renumbered, 16-bit ids, built on first use
-    int32_t sc_nlong = 0;       // ... its vertices with long lists
+    int32_t sc_nlong = -1;      // ... its vertices with long lists (-1: not counted yet)
     void *sc_report = nullptr;  // ... and its CTAs' reports (pinned)
     int sc_levels = 0;          // ... deepest level of its last launch
     void *ctl_host = nullptr;  // pinned copy of the batched engine's control block, written after each launch
@@ -275,7 +275,7 @@ void launch_bc(DeviceGraph &g, const int32_t *sources, int32_t k, const BcOption
                uint64_t *sigma_rows, double *delta_rows, int64_t ld, bool backward, cudaStream_t stream);
 // Small graphs, one CTA per source (smem_bc.cu): whether gu_bc / gu_sigma take it; bc
 // null: counts only.  Checks the sources on the device; synchronises.
-bool smem_bc_takes(const DeviceGraph &g, int32_t k, int32_t batch);
+bool smem_bc_takes(DeviceGraph &g, int32_t k, int32_t batch);
 void launch_smem_bc(DeviceGraph &g, const int32_t *sources, int32_t k, double *bc, int32_t *dist_rows,
                     uint64_t *sigma_rows, double *delta_rows, int64_t ld, cudaStream_t stream);
 // Throws GU_ERR_INVALID_ARGUMENT for a batch that gu_bc does not take.

@@ -46,6 +46,10 @@ namespace gu {
 constexpr int SC_MAX_THREADS = 1024;
 constexpr int SC_MAX_N = 8192;
 constexpr int64_t SC_MAX_M = 1 << 30;
+// Dense graphs (smem_bc_takes): above so many vertices, up to so many sources, above so
+// many entries.
+constexpr int SC_DENSE_N = 2500, SC_FEW = 16;
+constexpr int64_t SC_DENSE_M = 820000;
 constexpr int SC_LONG = 64;  // out-degree from which a warp takes a vertex
 constexpr unsigned SC_NONE = 0xFFFFu;
 
@@ -55,6 +59,8 @@ struct ScArgs {
     const uint16_t *__restrict__ newid;
     const uint16_t *__restrict__ oldid;
     int32_t n, nlong;                   // new ids below nlong have long lists
+    const int32_t *__restrict__ RT;     // in-edge offsets by old id
+    int32_t live;                       // vertices with in-edges
     const int32_t *__restrict__ sources;
     int32_t k;
     u64 *sigma_rows;     // k x ld, or null
@@ -206,6 +212,13 @@ __global__ void __launch_bounds__(SC_MAX_THREADS, 1) smem_bc_kernel(ScArgs a)
             }
             __syncthreads();
             if (!total) break;
+            // Nothing is left to reach (but the vertices with in-edges and the source): the
+            // level is the last and is not pushed.
+            if (fe + total >= a.live && fe + total >= a.live + (__ldg(a.RT + given) == __ldg(a.RT + given + 1))) {
+                ++level;
+                if (threadIdx.x == 0) lstart[level] = (uint16_t)(fe + total);
+                break;
+            }
             fs = fe;
             fe += total;
             flong = tlong;
@@ -399,12 +412,7 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
     for (size_t v = 0; v < n; ++v) newid[v] = (uint16_t)at[(size_t)key(v)]++;
     for (size_t v = 0; v < n; ++v) oldid[newid[v]] = (uint16_t)v;
     R2[0] = 0;
-    int32_t nlong = 0;
-    for (size_t i = 0; i < n; ++i) {
-        const int32_t d = R[oldid[i] + 1] - R[oldid[i]];
-        R2[i + 1] = R2[i] + d;
-        nlong += d >= SC_LONG;
-    }
+    for (size_t i = 0; i < n; ++i) R2[i + 1] = R2[i] + (R[oldid[i] + 1] - R[oldid[i]]);
     char *p = nullptr;
     GU_CUDA_CHECK(dev_malloc((void **)&p, bytes));
     g.extra_allocs.push_back(p);
@@ -416,7 +424,6 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
         g.R, g.C, g.n, dn, dold, reinterpret_cast<int32_t *>(p), reinterpret_cast<uint16_t *>(p + head));
     GU_CUDA_CHECK(cudaGetLastError());
     GU_CUDA_CHECK(cudaStreamSynchronize(stream));  // host goes out of scope
-    g.sc_nlong = nlong;
     g.sc_graph = p;
 }
 
@@ -426,9 +433,26 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
 // 256), R-MAT 13 k = 1024 1474 / 1676 (4335).  Above 8192 vertices the state does not
 // fit an SM.  A batch narrower than the request asks for passes, which only the batched
 // engine has.
-bool smem_bc_takes(const DeviceGraph &g, int32_t k, int32_t batch)
+// Where most lists are long a source reads nearly the whole adjacency here, once on the
+// way out and once on the way back, and a pass's sources share it there -- unless all is
+// reached within two levels (m / n squared over 12 n), where the way out ends early.
+// Times as fast as the batched engine, bc k = 1 / 40 / 1000: ER 8000 with 80 entries a
+// vertex 0.8 / 1.0 / 1.3, with 150 (1.2 M) 0.3 / 0.5 / 0.6, with 1000 0.8 / 2.0 / 2.4; ER
+// 4000 with 90 0.8 / 1.0 / 1.0, with 300 2.3 / 2.7 / 3.5; and with nearly all possible
+// entries ER 1000 0.5 / 0.7 / 1.3.
+bool smem_bc_takes(DeviceGraph &g, int32_t k, int32_t batch)
 {
     if (g.n < 1 || g.n > SC_MAX_N || g.m > SC_MAX_M || g.max_degree > SC_MAX_DEGREE || (batch != 0 && k > batch)) return false;
+    if (g.sc_nlong < 0) {
+        g.sc_nlong = 0;
+        for (int32_t v = 0; v < g.n; ++v) g.sc_nlong += g.host_R[v + 1] - g.host_R[v] >= SC_LONG;
+    }
+    const double n = (double)g.n, m = (double)g.m;
+    if (g.n > SC_DENSE_N) {
+        if (2 * g.sc_nlong > g.n && m * m < 12.0 * n * n * n && (k <= SC_FEW || g.m > SC_DENSE_M)) return false;
+    } else if (m > 550.0 * n && 8.0 * k * n < m) {
+        return false;
+    }
     for (const char *name : {"GU_BC_WORDS", "GU_BC_LEVEL_BUDGET_MB"}) {  // settings of the batched engine
         const char *s = std::getenv(name);
         if (s && *s) return false;
@@ -471,6 +495,8 @@ void launch_smem_bc(DeviceGraph &g, const int32_t *sources, int32_t k, double *b
     a.C = reinterpret_cast<const uint16_t *>(sg + r_bytes + 2 * id_bytes);
     a.n = g.n;
     a.nlong = g.sc_nlong;
+    a.RT = g.RT;
+    a.live = g.nlight + g.nmid + g.nwide + g.nheavy;
     a.sources = sources;
     a.k = k;
     a.sigma_rows = reinterpret_cast<u64 *>(sigma_rows);

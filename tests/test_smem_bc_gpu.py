@@ -153,3 +153,40 @@ def test_counts_that_wrap_to_zero(widths, what):
         for mine, ref in zip(*out):
             np.testing.assert_array_equal(np.isnan(mine), np.isnan(ref))
             np.testing.assert_allclose(mine, ref, rtol=RTOL, atol=0)  # infinities and NaN equal theirs
+
+
+@pytest.mark.parametrize("n,m,k,small", [(3000, 180000, 16, False), (3000, 180000, 17, True), (3000, 60000, 5, True),
+                                         (5000, 430000, 40, False), (900, 260000, 20, False), (900, 260000, 100, True),
+                                         (3000, 450000, 4, True)])
+def test_dense_graphs(n, m, k, small):
+    """Most lists long: few sources, and many on the largest graphs, go to the batched
+    engine, which reads the adjacency once for a pass's sources, unless two levels reach
+    everything.  Either engine's counts and betweenness are right."""
+    hg = gu.HostGraph.er(n, m, seed=1)
+    g = gu.Graph(hg)
+    srcs = gu.sources(n, k, seed=2)
+    s = torch.as_tensor(srcs, device="cuda")
+    sig = torch.empty((k, n), dtype=torch.int64, device="cuda")
+    bc = torch.empty(n, dtype=torch.float64, device="cuda")
+    g.sigma(s, sig)
+    assert (g.level_profile() == []) == small
+    np.testing.assert_array_equal(sig.cpu().numpy().view(np.uint64), oracle.sigma_multi(hg.R, hg.C, n, srcs, nthreads=8)[1])
+    g.bc(s, bc)
+    assert (g.level_profile() == []) == small
+    np.testing.assert_allclose(bc.cpu().numpy(), oracle.bc(hg.R, hg.C, n, srcs, nthreads=8), rtol=RTOL, atol=0)
+
+
+def test_searches_that_reach_everything():
+    """The last level is not pushed once all vertices with in-edges, and the source, are
+    reached: sources without in-edges, with all others on one level, one vertex short of
+    everything, a vertex that only another source reaches, and a single vertex."""
+    n = 70
+    a, b = np.meshgrid(np.arange(n), np.arange(n))
+    check(gu.HostGraph.from_edges(n, a.ravel(), b.ravel()), np.arange(n, dtype=np.int32))  # complete
+    below = a.ravel() < b.ravel()
+    check(gu.HostGraph.from_edges(n, a.ravel()[below], b.ravel()[below], symmetric=False), np.arange(n, dtype=np.int32), True)
+    for extra in ([], [(68, 69)], [(69, 0)], [(0, 69), (69, 68)]):
+        u = np.array([0] * 30 + [1 + i % 30 for i in range(200)] + [e[0] for e in extra])
+        v = np.array(list(range(1, 31)) + [31 + (7 * i) % 38 for i in range(200)] + [e[1] for e in extra])
+        check(gu.HostGraph.from_edges(n, u, v, symmetric=False), np.array([0, 1, 30, 31, 68, 69], np.int32), True)
+    check(gu.HostGraph(np.zeros(2, np.int32), np.zeros(0, np.int32), 1), np.array([0], np.int32))
