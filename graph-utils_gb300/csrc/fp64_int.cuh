@@ -41,15 +41,19 @@ __host__ __device__ __forceinline__ u64 mantissa_quotient(u64 ma, u64 mb, unsign
 __host__ __device__ __forceinline__ u64 quotient_bits(u64 a, u64 b, unsigned r0)
 {
     constexpr u64 M = (1ull << 52) - 1;
-    const u64 q = mantissa_quotient((a & M) | (M + 1), (b & M) | (M + 1), r0);
+    const u64 ma = (a & M) | (M + 1), mb = (b & M) | (M + 1), q = mantissa_quotient(ma, mb, r0);
     const int lt1 = q < (1ull << 62);
-    const u64 m = (q + (lt1 ? 256 : 512)) >> (lt1 ? 9 : 10);  // [2^52, 2^53]
+    // the mantissa is h or h + 1: which one, the exact remainder from the middle between
+    // them tells (in 64 bits, wrapping; below 2^54, and never 0: a quotient of two
+    // mantissas of 53 bits does not have 54)
+    const u64 h = q >> (lt1 ? 9 : 10);
+    const long long past = (long long)((ma << (lt1 ? 54 : 53)) - (2 * h + 1) * mb);
+    const u64 m = h + (past > 0);  // [2^52, 2^53]
     return m + ((u64)((int)(a >> 52) - (int)(b >> 52) + 1022 - lt1) << 52);
 }
 
-// a / b for a >= 1 and 1 <= b < 2^64 (so that the quotient of a finite a is normal),
-// rounded to nearest but for quotients within 2^-9 of a unit of the rounding boundary;
-// anything else goes through the division itself.
+// a / b, rounded to nearest as the division is: for a >= 1 and 1 <= b < 2^64 (so that the
+// quotient of a finite a is normal); anything else goes through the division itself.
 __device__ __forceinline__ double quotient(double a, double b)
 {
     const u64 x = (u64)__double_as_longlong(a), y = (u64)__double_as_longlong(b);
