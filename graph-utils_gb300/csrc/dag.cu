@@ -31,6 +31,7 @@ constexpr int CLOSURE_CHUNK = 4096;               // columns per warp step: 16 b
 // lists short enough for eight lanes.
 constexpr int REACH_MAX_LEVELS = 96;
 constexpr int32_t REACH_MAX_IN_DEGREE = 2048;
+constexpr int REACH_LEVEL_VERTICES = 1000;  // vertices per level at least, where out-degrees are low
 // Rows kept at once: the closure runs in column blocks of at most this many bytes
 // of rows (n = 65536 fits one block; a block costs one pass over the levels, about
 // 3 us each, so narrower blocks that would stay in L2 cost more than they save).
@@ -581,6 +582,14 @@ bool launch_dag_reach(DeviceGraph &g, const int32_t *sources, int32_t k, unsigne
     const char *env = std::getenv("GU_AUTO_LOCAL");
     if (env && env[0] == '0') return false;
     if (!g.directed || g.n < 1 || g.n > TOPO_MAX_N || g.max_in_degree > REACH_MAX_IN_DEGREE) return false;
+    // Graphs of low out-degree have the per-source engine, which runs two sources per SM at
+    // about a level's cost here each: the order pays where there is more to a level than
+    // that.  Call times in us, by the order / that engine, k = 100 and 600: binary out-tree of
+    // 60000 vertices 77 / 51 and 159 / 64; DAG of 20000, m = n 69 / 50 and 130 / 72, of
+    // 50000, m = 2 n 89 / 80 and 194 / 96; 90 layers of 500, m = 4 n 337 / 287 and 878 / 574.
+    const bool low = g.max_degree <= LOCAL_MAX_DEGREE;
+    if (low && g.m < 3 * (int64_t)g.n) return false;
+    const int max_levels = low ? std::min(REACH_MAX_LEVELS, g.n / REACH_LEVEL_VERTICES) : REACH_MAX_LEVELS;
     char *ws = nullptr;
     const int W = msbfs_words_for(k);
     // The order costs about as much to build as the searches that it replaces save in one
@@ -589,7 +598,7 @@ bool launch_dag_reach(DeviceGraph &g, const int32_t *sources, int32_t k, unsigne
     if (g.topo.state == TopoPlan::UNBUILT && g.topo.asked++ == 0) return false;
     try {
         const size_t need = WS_CONTROL_BYTES + sizeof(u64) * (size_t)g.n * W;
-        if (!ensure_topo(g, REACH_MAX_LEVELS, need, st)) return false;
+        if (!ensure_topo(g, max_levels, need, st)) return false;
         ws = (char *)g.ws.get(need);
     } catch (const gu_error &e) {
         if (e.code == GU_ERR_OUT_OF_MEMORY) return false;

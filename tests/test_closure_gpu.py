@@ -134,7 +134,9 @@ def test_orders_that_are_not_used_are_not_kept(levels):
     n = 20000
     v = np.arange(n)
     u = v[(v % levels != levels - 1) & (v < n - 1)]
-    chains = gu.HostGraph.from_edges(n, u, u + 1, symmetric=False)
+    ends = np.setdiff1d(v, u)[:20] if levels < 1000 else np.full(20, n - 1) - np.arange(20)
+    # (a hub in front of some vertices, so that the graph is not one of low out-degree)
+    chains = gu.HostGraph.from_edges(n + 1, np.concatenate([u, np.full(20, n)]), np.concatenate([u + 1, ends]), symmetric=False)
     ring = gu.HostGraph.from_edges(n, v, (v + 1) % n, symmetric=False)
     order_bytes = 4 * (6 * n + 3 + 2 * (n - n // levels - 1))
     s = torch.arange(0, n, 2501, dtype=torch.int32, device="cuda")
@@ -154,9 +156,35 @@ def test_orders_that_are_not_used_are_not_kept(levels):
             counts_are_right()
         kept = g.device_bytes() - before  # and what the workspace grew by, at most 0.35 MB here
         assert (kept >= order_bytes) == (hg is chains and levels <= 96)
-        sizes = torch.empty(n, dtype=torch.int64, device="cuda")
+        sizes = torch.empty(hg.n, dtype=torch.int64, device="cuda")
         g.dag_reach(sizes)
         np.testing.assert_array_equal(sizes.cpu().numpy()[at], want - 1)
         if hg is ring:  # the search's workspace, not the closure's rows (50 MB)
             assert g.device_bytes() - before < 10e6
         counts_are_right()
+
+
+def test_low_degree_graphs_stay_with_the_search():
+    """Trees and graphs of few vertices per level, out-degree up to 16: no order is built
+    for their reachable counts; one of many vertices per level has one from the second
+    call on.  The counts are right either way."""
+    n = 20000
+    i = np.arange(1, n)
+    rng = np.random.default_rng(3)
+    layers = [np.concatenate([l * 200 + np.repeat(np.arange(200), 4) for l in range(90)]),
+              np.concatenate([(l + 1) * 200 + rng.integers(0, 200, 800) for l in range(90)])]
+    wide = [np.repeat(np.arange(15000), 5), 15000 + rng.integers(0, 5000, 75000)]
+    for u, v, ordered in (((i - 1) // 2, i, False), (layers[0], layers[1], False), (wide[0], wide[1], True)):
+        hg = gu.HostGraph.from_edges(n, u, v, symmetric=False)
+        g = gu.Graph(hg)
+        srcs = gu.sources(n, 9, seed=1)
+        s = torch.as_tensor(srcs, device="cuda")
+        want = (oracle.bfs_multi(hg.R, hg.C, n, srcs)[0] != gu.UNREACHABLE).sum(1)
+        cnt = torch.full((9,), -1, dtype=torch.int64, device="cuda")
+        sizes = []
+        for _ in range(3):
+            g.reach(s, cnt)
+            np.testing.assert_array_equal(cnt.cpu().numpy(), want)
+            sizes.append(g.device_bytes())
+        # the order is 24 bytes a vertex and 8 an edge; the workspace grows by less here
+        assert (sizes[2] - sizes[0] >= 24 * n + 8 * hg.m) == ordered
