@@ -191,15 +191,15 @@ def test_without_memory_for_its_tables(n, after):
 
 
 def test_direction_counts_all_frontier_edges():
-    """1024 neighbours of the source, in the first words of the bitmap, with 40 out-edges
-    each: their edges are summed by other warps than find them, and all 40960 count.  The
-    second level is then searched bottom-up (40960^2 against 6975 vertices left x 200000
-    edges), and so is the third; with part of the edges the second would be top-down, as
-    the first and the last are, which find one and twenty vertices' neighbours."""
+    """1024 neighbours of the source, in the first words of the bitmap, with 64 out-edges
+    each: their edges are summed by other warps than find them, and all 65536 count.  The
+    second level is then searched bottom-up (65536^2 against twice 6975 vertices left x
+    200000 edges) and finds all of them, and so is the third, which finds nothing; with
+    part of the edges the second would be top-down, as the first is."""
     rng = np.random.default_rng(4)
     n, mid, end = 16000, 1025, 8000
-    u = np.concatenate([np.zeros(1024, np.int64), np.repeat(np.arange(1, mid), 40), rng.integers(mid, end, 158000)])
-    v = np.concatenate([np.arange(1, mid), rng.integers(mid, end, 40960), rng.integers(mid, end, 158000)])
+    u = np.concatenate([np.zeros(1024, np.int64), np.repeat(np.arange(1, mid), 64), rng.integers(mid, end, 133440)])
+    v = np.concatenate([np.arange(1, mid), rng.integers(mid, end, 65536), rng.integers(mid, end, 133440)])
     order = np.argsort(u, kind="stable")  # parallel edges stay: the counts are exact
     R = np.concatenate([[0], np.cumsum(np.bincount(u, minlength=n))])
     hg = gu.HostGraph(R, v[order], n, directed=True)
@@ -207,4 +207,4 @@ def test_direction_counts_all_frontier_edges():
     got = rows(g, [0])
     td, bu, ml = g.last_launch()[1:]
     np.testing.assert_array_equal(got, oracle.bfs_multi(hg.R, hg.C, n, [0])[0])
-    assert g.level_profile() == [] and (td, bu, ml) == (2, 2, 3)
+    assert g.level_profile() == [] and (td, bu, ml) == (1, 2, 2)
