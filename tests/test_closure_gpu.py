@@ -188,3 +188,17 @@ def test_low_degree_graphs_stay_with_the_search():
             sizes.append(g.device_bytes())
         # the order is 24 bytes a vertex and 8 an edge; the workspace grows by less here
         assert (sizes[2] - sizes[0] >= 24 * n + 8 * hg.m) == ordered
+
+
+@pytest.mark.parametrize("n", [3000, 9000])
+def test_stars_and_hubs(n):
+    """A hub's successors are ORed one after another: a graph that is little else goes to
+    the search from every vertex; the sizes are the same either way."""
+    i = np.arange(1, n)
+    for u, v in ((i * 0, i), (np.concatenate([i * 0, i[:-1]]), np.concatenate([i, i[1:]])), (i * 0, i // 2 * 2)):
+        keep = u != v
+        hg = gu.HostGraph.from_edges(n, u[keep], v[keep], symmetric=False)
+        counts, tot = closure(hg)
+        ref, rtot = oracle.dag_reach_counts(hg.R, hg.C, hg.n)
+        np.testing.assert_array_equal(counts, ref)
+        assert tot == rtot
