@@ -437,9 +437,10 @@ static void ensure_renumbered(DeviceGraph &g, cudaStream_t stream)
 // way out and once on the way back, and a pass's sources share it there -- unless all is
 // reached within two levels (m / n squared over 12 n), where the way out ends early.
 // Times as fast as the batched engine, bc k = 1 / 40 / 1000: ER 8000 with 80 entries a
-// vertex 0.8 / 1.0 / 1.3, with 150 (1.2 M) 0.3 / 0.5 / 0.6, with 1000 0.8 / 2.0 / 2.4; ER
-// 4000 with 90 0.8 / 1.0 / 1.0, with 300 2.3 / 2.7 / 3.5; and with nearly all possible
-// entries ER 1000 0.5 / 0.7 / 1.3.
+// vertex 0.5 / 0.7 / 0.9, with 150 (1.2 M) 0.3 / 0.5 / 0.6, with 1000 0.8 / 2.0 / 2.4; ER
+// 4000 with 90 0.6 / 0.8 / 0.8, with 150 0.6 / 0.8 / 0.8 (k = 150 and 300, whole waves of
+// CTAs: 1.3), with 300 2.3 / 2.7 / 3.5; and with nearly all possible entries ER 1000 0.5 /
+// 0.7 / 1.3.
 bool smem_bc_takes(DeviceGraph &g, int32_t k, int32_t batch)
 {
     if (g.n < 1 || g.n > SC_MAX_N || g.m > SC_MAX_M || g.max_degree > SC_MAX_DEGREE || (batch != 0 && k > batch)) return false;
@@ -449,7 +450,9 @@ bool smem_bc_takes(DeviceGraph &g, int32_t k, int32_t batch)
     }
     const double n = (double)g.n, m = (double)g.m;
     if (g.n > SC_DENSE_N) {
-        if (2 * g.sc_nlong > g.n && m * m < 12.0 * n * n * n && (k <= SC_FEW || g.m > SC_DENSE_M)) return false;
+        if (2 * g.sc_nlong > g.n && m * m < 12.0 * n * n * n &&
+            (k <= SC_FEW || g.m > SC_DENSE_M || (m > 100.0 * n && (k <= 100 || k > 400))))
+            return false;
     } else if (m > 550.0 * n && 8.0 * k * n < m) {
         return false;
     }

@@ -155,7 +155,8 @@ def test_counts_that_wrap_to_zero(widths, what):
             np.testing.assert_allclose(mine, ref, rtol=RTOL, atol=0)  # infinities and NaN equal theirs
 
 
-@pytest.mark.parametrize("n,m,k,small", [(3000, 180000, 16, False), (3000, 180000, 17, True), (3000, 60000, 5, True),
+@pytest.mark.parametrize("n,m,k,small", [(3000, 120000, 16, False), (3000, 120000, 17, True), (3000, 60000, 5, True),
+                                         (3000, 180000, 100, False), (3000, 180000, 101, True), (3000, 180000, 401, False),
                                          (5000, 430000, 40, False), (900, 260000, 20, False), (900, 260000, 100, True),
                                          (3000, 450000, 4, True)])
 def test_dense_graphs(n, m, k, small):
