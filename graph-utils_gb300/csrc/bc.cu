@@ -378,9 +378,10 @@ __device__ __forceinline__ void finish_delta(const BcArgs &a, size_t o, double S
 // terms one at a time in CSR order (a successor's list holds a source at most
 // once, and successive lists are separated by __syncwarp), so the sums are the
 // sequential CSR-order sums.  The lists of SUCC successors are made together, a lane per
-// 32-bit word of a mask (a successor at a time, by ranks, cost 72 instructions each: R-MAT18, 1024 sources, levels 1 / 2 / 3 took 2.34 / 6.14 / 3.85 ms, now 1.58 /
-// 5.48 / 3.13; six or eight rounds of loads in flight instead of four are slower, 5.63
-// and 6.07 ms on level 2).
+// 32-bit word of a mask (a successor at a time, by ranks, cost 72 instructions each:
+// R-MAT18, 1024 sources, levels 1 / 2 / 3 took 2.34 / 6.14 / 3.85 ms, now 1.58 / 5.48 /
+// 3.13; six or eight rounds of loads in flight instead of four are slower, 5.63 and 6.07
+// ms on level 2).
 template <int NQ>
 struct SumStage {
     double acc[64 * NQ];

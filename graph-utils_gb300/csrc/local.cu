@@ -13,9 +13,9 @@
 // live in shared memory, a thread expands the whole adjacency list of a low-degree
 // vertex with four claims in flight, and appends are warp-aggregated shared
 // atomics.  A frontier larger than the shared queue ends the launch with a flag and
-// the caller reruns the search on the batched engine.  Rows mode claims vertices in the distance row itself; the counting
-// modes (diameter, reachability) claim them in a per-CTA visited bitmap and
-// write no rows.
+// the caller reruns the search on the batched engine.  Rows mode claims vertices in the
+// distance row itself; the counting modes (diameter, reachability) claim them in a
+// per-CTA visited bitmap and write no rows.
 //
 // The adjacency is read from a padded copy (ELL: the neighbours of v in CSR
 // order at v * width, width 4, 8 or 16, padded with -1), built on the graph's

@@ -2056,9 +2056,10 @@ static int queue_blocks_per_sm()
     return b;
 }
 
-// Estimated work of k sources of a request: passes over the vertices' words, over the
-// adjacency (a DAG's vertices are met again at several distances), the rows, and the
-// levels' fixed part.  The weights were varied by factors of two and more on four
+// Estimated work of k sources of a request, in units of the time in which a CTA moves a
+// byte of a row: the levels' fixed part, passes over the vertices' words (per vertex) and
+// over the adjacency (per entry; ten times on a DAG, whose vertices are met again at
+// several distances), and the rows (two passes over four bytes).  The weights were varied by factors of two and more on four
 // request sets: the launch stayed within 2 % of the best but for cheaper DAGs or
 // dearer adjacencies (5-10 % longer).
 static double queue_weight(const MsQueueRequest &r, int32_t k)

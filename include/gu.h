@@ -196,7 +196,9 @@ gu_status gu_graph_launch_times(gu_graph g, int max_entries, double *kernel_seco
  * 11 bc accumulation and per-source rows, 12 a forward level's bitmap cleared),
  * vertices and out-edges of the frontier it expanded (batched search only; 0 for
  * BC), and the time the slowest CTA finished it, in ms from the end of entry 0.
- * No reference counterpart (the reference times whole calls only). */
+ * The shared-memory engines (small graphs) and the counts by a DAG's order keep no
+ * timeline: no entries.  No reference counterpart (the reference times whole calls
+ * only). */
 gu_status gu_graph_level_profile(gu_graph g, int max_entries, int32_t *batch, int32_t *level, int32_t *kind,
                                  int64_t *frontier_vertices, int64_t *frontier_edges, double *t_ms, int *count);
 
@@ -253,7 +255,9 @@ gu_status gu_graph_set_tuning(gu_graph g, const gu_tuning *t);
  * scan_based,shuffle_based}_setup (linear_with_atomics.cuh:14,
  * edge_parallel.cuh:13, warp_based.cuh:15, CTA_warp.cuh:15, scan_based.cuh:15,
  * shuffle_based.cuh:16), which return the rows of the last #SM sources only;
- * this call returns every row. */
+ * this call returns every row.  A source out of range gives
+ * GU_ERR_INVALID_ARGUMENT; where the batched engine runs (any named variant but
+ * PLAIN, AUTO on larger graphs) the other sources' rows are written then. */
 gu_status gu_bfs(gu_graph g, int variant, const int32_t *sources_dev, int32_t k, int32_t *dist_dev, int64_t ld,
                  void *stream);
 gu_status gu_bfs_host(gu_graph g, int variant, const int32_t *sources_host, int32_t k, int32_t *dist_host,
