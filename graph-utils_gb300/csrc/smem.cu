@@ -622,14 +622,14 @@ static SbConfig sb_config(const DeviceGraph &g, int S, int threads)
 // engine / the engine AUTO took before, k sources:
 //   n <= 16384, always: one CTA per source keeps its advantage at any k (R-MAT 12
 //     k = 300 50 / 360, R-MAT 14 k = 150 59 / 154, k = 1500 279 / 919, ER 2000
-//     k = 512 74 / 180).  Out-degrees up to 16 have an engine of their own (local.cu),
+//     k = 512 71 / 180).  Out-degrees up to 16 have an engine of their own (local.cu),
 //     which is level from n = 6400, k = 256 (524 / 488) down and behind elsewhere
 //     (128 x 128 grid k = 1 507 / 649, k = 256 665 / 784); above, it is ahead
 //     (256 x 256 grid 1477 / 1277).
 //   n <= 32768: up to one source per SM and k m = 140 M (R-MAT 15 k = 150 90 / 174,
-//     ER 30000 k = 150 98 / 143; k = 300 196 / 254, but behind on denser graphs).
+//     ER 30000 k = 150 101 / 143; k = 300 196 / 254, but behind on denser graphs).
 //   above, by k m, the work that the batched engine shares among the sources: up to
-//     60 M (R-MAT 16 k = 32 70 / 143, ER 100000 k = 30 131 / 143; ER 65000 k = 80 226 /
+//     60 M (R-MAT 16 k = 32 70 / 143, ER 100000 k = 30 98 / 143; ER 65000 k = 80 226 /
 //     157), with four CTAs a source at least (a DAG of 60000 vertices and 26 levels,
 //     counts, k = 100, one CTA a source: 451 / 305), and beyond 131072 vertices, where
 //     a source needs eight CTAs, up to 8 sources (R-MAT 18 k = 8 115 / 153, k = 16 179 /
